@@ -348,6 +348,7 @@ int sck_plan_create(const sck_system_desc* d, int32_t batch, int32_t mode, sck_p
   p->NP = np < 1 ? 1 : np;
   p->field = (d->n == 1 && d->h64[0] != 0.0) ? 1 : 0;
   p->spec = find_spec(p);
+  p->word_spec = find_word_spec(p);
   if (mode == SCK_MODE_QUAD) {
     std::string why;
     if (!quad_ok(p, &why)) {
@@ -390,6 +391,7 @@ int sck_plan_tune(sck_plan* plan, int32_t specialised, int64_t l2_budget_bytes, 
     return fail(SCK_ERR_INVALID, "null plan or negative budget");
   if (resident_limit_bytes > kResidentMax) return fail(SCK_ERR_INVALID, "resident limit above 220 KiB of shared memory");
   plan->spec = (specialised || plan->mode == SCK_MODE_QUAD) ? find_spec(plan) : 0;   // interleaved: always
+  plan->word_spec = specialised ? find_word_spec(plan) : 0;
   plan->kernel_kind = specialised >= 3 ? 3 : (specialised >= 2 ? 2 : 1);
   plan->l2_budget = l2_budget_bytes;
   plan->resident_limit = resident_limit_bytes;
@@ -546,6 +548,7 @@ static int class_launch(const sck_plan* plan, const sck_buffers* buf, const void
     return launch_quad_class(plan, buf, colour, alpha, s);
   }
   Common c = make_common(plan, buf, src);
+  if (plan->word_spec && colour >= 0 && src == buf->spins) return launch_word_class(plan, c, colour, alpha, s);
   if (is_bitwise(plan->mode)) return launch_bitwise_class(plan, c, colour, alpha, s);
   return launch_class(plan, c, colour, alpha, s);
 }

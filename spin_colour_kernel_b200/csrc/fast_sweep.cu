@@ -173,8 +173,8 @@ static bool matches(const sck_plan* p) {
   return true;
 }
 
-int find_spec(const sck_plan* p) {
-  if (p->mode != SCK_MODE_INT8 && p->mode != SCK_MODE_F32 && p->mode != SCK_MODE_QUAD) return 0;
+// Id of the compile-time table that equals the plan's bond lists, or 0.
+int match_lattice(const sck_plan* p) {
   if (matches<Lat_square_1>(p)) return Lat_square_1::id;
   if (matches<Lat_triangular_1>(p)) return Lat_triangular_1::id;
   if (matches<Lat_sc_1>(p)) return Lat_sc_1::id;
@@ -182,6 +182,11 @@ int find_spec(const sck_plan* p) {
   if (matches<Lat_bcc_1_2>(p)) return Lat_bcc_1_2::id;
   if (matches<Lat_fcc_1>(p)) return Lat_fcc_1::id;
   return 0;
+}
+
+int find_spec(const sck_plan* p) {
+  if (p->mode != SCK_MODE_INT8 && p->mode != SCK_MODE_F32 && p->mode != SCK_MODE_QUAD) return 0;
+  return match_lattice(p);
 }
 
 // ------------------------------------------------------------------------------------------- host: launches
@@ -228,8 +233,8 @@ static bool periodic_box(const sck_plan* plan) {
   return g.dim == 2 || (g.per[2] && g.L3 >= Lat::reach);
 }
 
-int spec_periodic_box(const sck_plan* plan) {
-  switch (plan->spec) {
+int lattice_periodic_box(const sck_plan* plan, int id) {
+  switch (id) {
     case Lat_square_1::id: return periodic_box<Lat_square_1>(plan) ? 1 : 0;
     case Lat_triangular_1::id: return periodic_box<Lat_triangular_1>(plan) ? 1 : 0;
     case Lat_sc_1::id: return periodic_box<Lat_sc_1>(plan) ? 1 : 0;
@@ -239,6 +244,8 @@ int spec_periodic_box(const sck_plan* plan) {
     default: return 0;
   }
 }
+
+int spec_periodic_box(const sck_plan* plan) { return lattice_periodic_box(plan, plan->spec); }
 
 template <class Lat, class P>
 static void launch_lat(const sck_plan* plan, const P& p, dim3 grid, cudaStream_t s) {

@@ -39,6 +39,16 @@ struct Common {
 // no site of the class. Along a row the colour has period P and each colour of the row appears at most once per
 // period, so stepping the per-factor residues through one period finds it.
 __device__ __forceinline__ int first_class_x(const Common& c, int colour, int alpha, int y, int z) {
+  if (c.col.r == 1) {                  // one cyclic factor: the colour is its residue
+    const uint32_t v = (uint32_t)(c.col.K[0][1] * y + c.col.K[0][2] * z + c.col.o[alpha][0]);
+    int g = (int)(v - fdiv(v, c.fd_m[0]) * (uint32_t)c.col.m[0]);
+    for (int q = 0; q < c.P; ++q) {
+      if (g == colour) return q;
+      g += c.col.K[0][0];
+      if (g >= c.col.m[0]) g -= c.col.m[0];
+    }
+    return c.g.L1;
+  }
   int g[SCK_MAX_FACTORS];
 #pragma unroll
   for (int r = 0; r < SCK_MAX_FACTORS; ++r) {
@@ -120,6 +130,7 @@ struct sck_plan {
   int Z, Z1, NP, field;
   int ising_lut;   // Ising chain with the host-built exp table (INT8, F32 with n = 1, PACKED)
   int spec;        // id of the matching compile-time lattice table (lattices.h), 0 = generic kernels
+  int word_spec;   // the same for word storage (words.cu), 0 = the kernels of sweep.cu and bitwise.cu
   int kernel_kind; // specialised class kernels: 1 lattice, 2 segment (segment.cu), 3 tile (tile.cu) where eligible
   long long l2_budget;  // bytes of L2 the group pipeline may fill
   long long resident_limit;  // largest replica (bytes) whose sweeps run resident in shared memory; 0 = never
@@ -159,7 +170,11 @@ int launch_topological_charge(const sck_plan* plan, const float* spins, const in
 int launch_pack(const sck_plan* plan, const int8_t* spins, int32_t* words, cudaStream_t s);
 int launch_unpack(const sck_plan* plan, const int32_t* words, const int8_t* mask, int8_t* spins, cudaStream_t s);
 int launch_advance(int64_t* state, int n, cudaStream_t s);
+int match_lattice(const sck_plan* plan);
+int lattice_periodic_box(const sck_plan* plan, int id);
 int find_spec(const sck_plan* plan);
+int find_word_spec(const sck_plan* plan);
+int launch_word_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s);
 size_t resident_bytes(const sck_plan* plan);
 int launch_resident(const sck_plan* plan, const Common& c, int n_sweeps, cudaStream_t s);
 int launch_spec_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s);
