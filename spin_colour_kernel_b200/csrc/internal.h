@@ -160,7 +160,8 @@ int check_observables_request(const sck_plan* plan, int storage, int batch);
 int made_wait_timeouts(unsigned long long* count);
 int made_set_wait_limit(long long polls);   // polls before the tensor-core GEMM's stage waits give up   // bounded waits of the learned proposal's kernels that gave up
 int launch_observables(const sck_plan* plan, const void* spins, int storage, int batch, const int8_t* mask,
-                       const float* k1, double* E, double* M, void* workspace, cudaStream_t s);
+                       const float* k1, double* E, double* M, void* workspace, cudaStream_t s,
+                       int scratch_blocks = 0);
 int launch_observables_finish(const double* partial, int B, int blocks_per_rep, int b, int n, double* E, double* M,
                               cudaStream_t s);
 int launch_observables_fold(const sck_plan* plan, int batch, const double* E, const double* M, double n_active,
@@ -174,6 +175,9 @@ int match_lattice(const sck_plan* plan);
 int lattice_periodic_box(const sck_plan* plan, int id);
 int find_spec(const sck_plan* plan);
 int find_word_spec(const sck_plan* plan);
+bool word_columns_ok(const sck_plan* plan);
+int word_column_blocks(const sck_plan* plan, int batch);
+int launch_word_columns(const sck_plan* plan, const ObsParams& p, cudaStream_t s);
 int launch_word_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s);
 size_t resident_bytes(const sck_plan* plan);
 int launch_resident(const sck_plan* plan, const Common& c, int n_sweeps, cudaStream_t s);

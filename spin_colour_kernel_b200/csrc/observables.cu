@@ -9,7 +9,7 @@
 #include <string>
 
 #include "internal.h"
-#include "spec.cuh"
+#include "words.cuh"
 
 namespace sck {
 
@@ -414,14 +414,29 @@ static int launch_obs_tile(const sck_plan* plan, const ObsParams& p, cudaStream_
   }
 }
 
-// Sum the partials of every replica in block order; E[r] and M[r][alpha][k] (B x b x n).
-__global__ void observables_finish(const double* __restrict__ partial, int B, int blocks_per_rep, int b, int n,
-                                   double* __restrict__ E, double* __restrict__ M) {
-  const int rep = blockIdx.x * blockDim.y + threadIdx.y;
-  const int v = threadIdx.x;
-  if (rep >= B || v >= 1 + b * n) return;
+// Sum the partials of every replica in a fixed order; E[r] and M[r][alpha][k] (B x b x n). One block per replica:
+// FINISH_LANES threads per value each add every FINISH_LANES-th partial (independent, coalesced loads), then meet in
+// shared memory. Bound by load latency: one thread per value adding all partials in turn took 22 us at 296 partials
+// of 128 replicas, this takes 4.
+constexpr int FINISH_LANES = 8;
+
+__global__ void __launch_bounds__(OBS_VALUES * FINISH_LANES)
+    observables_finish(const double* __restrict__ partial, int blocks_per_rep, int b, int n, double* __restrict__ E,
+                       double* __restrict__ M) {
+  __shared__ double red[FINISH_LANES][OBS_VALUES];
+  const int rep = blockIdx.x, v = threadIdx.x, l = threadIdx.y;
+  const bool live = v < 1 + b * n;
   double x = 0.0;
-  for (int i = 0; i < blocks_per_rep; ++i) x += partial[((size_t)rep * blocks_per_rep + i) * OBS_VALUES + v];
+  if (live) {
+    const double* src = partial + (size_t)rep * blocks_per_rep * OBS_VALUES + v;
+#pragma unroll 4
+    for (int i = l; i < blocks_per_rep; i += FINISH_LANES) x += src[(size_t)i * OBS_VALUES];
+  }
+  red[l][v] = x;
+  __syncthreads();
+  if (l != 0 || !live) return;
+#pragma unroll
+  for (int i = 1; i < FINISH_LANES; ++i) x += red[i][v];
   if (v == 0) {
     if (E != nullptr) E[rep] = x;
   } else if (M != nullptr) {
@@ -454,10 +469,22 @@ static int obs_blocks_words(const sck_plan* plan, int batch) {
   return want < per_rep ? (want < 1 ? 1 : want) : per_rep;
 }
 
-int obs_launch_blocks(const sck_plan* plan, int storage, int batch) {
+static bool obs_columns(const sck_plan* plan, int storage) {
+  return storage == SCK_MODE_PACKED && plan->word_spec != 0 && word_columns_ok(plan);
+}
+
+// Slots per replica a call without a workspace is accepted by: the launch's own count, except that the column
+// kernel, which runs with as many blocks as there is room for, is held to the count of the kernels it stands for.
+static int obs_scratch_slots(const sck_plan* plan, int storage, int batch) {
   if (storage == SCK_MODE_QUAD) return quad_obs_blocks(plan);
   if (obs_words_ok(plan, storage)) return obs_blocks_words(plan, batch);
   return obs_tiled(plan, storage) ? plan->geom.L2 / OBS_TY : obs_blocks_generic(plan, batch);
+}
+
+int obs_launch_blocks(const sck_plan* plan, int storage, int batch) {
+  if (storage == SCK_MODE_QUAD) return quad_obs_blocks(plan);
+  if (obs_columns(plan, storage)) return word_column_blocks(plan, batch);
+  return obs_scratch_slots(plan, storage, batch);
 }
 
 // Partial sums per replica a caller's workspace must hold: the largest count any storage and tuning of this plan
@@ -468,6 +495,7 @@ int obs_blocks_per_rep(const sck_plan* plan, int batch) {
   if (tile > most) most = tile;
   if (plan->mode == SCK_MODE_QUAD && quad_obs_blocks(plan) > most) most = quad_obs_blocks(plan);
   if (obs_words_ok(plan, SCK_MODE_PACKED) && obs_blocks_words(plan, batch) > most) most = obs_blocks_words(plan, batch);
+  if (word_columns_ok(plan) && word_column_blocks(plan, batch) > most) most = word_column_blocks(plan, batch);
   return most;
 }
 
@@ -568,19 +596,6 @@ int launch_topological_charge(const sck_plan* plan, const float* spins, const in
 // the same site energy -1/2 s v - h s as observables_kernel, written to the same partial slots.
 constexpr int kWordObsBonds = 8;
 
-// Number of threads of the warp whose mask has bit `lane` set, for every lane at once: the warp's 32 masks as a
-// 32 x 32 bit matrix (row = thread, column = bit) transposed by exchanging off-diagonal blocks of 16, 8, 4, 2 and
-// 1 across lane ^ s, then the popcount of the lane's column.
-__device__ __forceinline__ unsigned warp_lane_counts(uint32_t x, int lane) {
-  const uint32_t lo[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-  for (int i = 0, sh = 16; i < 5; ++i, sh >>= 1) {
-    const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, sh);
-    x = (lane & sh) ? ((x & ~lo[i]) | ((y & ~lo[i]) >> sh)) : ((x & lo[i]) | ((y & lo[i]) << sh));
-  }
-  return (unsigned)__popc(x);
-}
-
 __global__ void __launch_bounds__(256) observables_words_kernel(const __grid_constant__ ObsParams p) {
   const Geometry& g = p.g;
   const int w = blockIdx.y;
@@ -672,8 +687,9 @@ static bool obs_words_ok(const sck_plan* plan, int storage) {
   return true;
 }
 
+// `scratch_blocks` > 0 bounds the partial-sum slots per replica (the column kernel runs with any number of blocks).
 int launch_observables(const sck_plan* plan, const void* spins, int storage, int batch, const int8_t* mask,
-                       const float* k1, double* E, double* M, void* workspace, cudaStream_t s) {
+                       const float* k1, double* E, double* M, void* workspace, cudaStream_t s, int scratch_blocks) {
   if (storage == SCK_MODE_QUAD) return launch_quad_observables(plan, spins, batch, k1, E, M, workspace, s);
   ObsParams p;
   p.g = plan->geom;
@@ -688,6 +704,8 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
   // float32 storage of a tiled-geometry system with its lattice table on: bands of OBS_TY rows
   const bool tile = obs_tiled(plan, storage);
   p.blocks_per_rep = obs_launch_blocks(plan, storage, batch);
+  if (scratch_blocks > 0 && p.blocks_per_rep > scratch_blocks && obs_columns(plan, storage))
+    p.blocks_per_rep = scratch_blocks;
   p.fd_plane = make_fastdiv((uint32_t)plan->geom.plane);
   p.fd_L1 = make_fastdiv((uint32_t)plan->geom.L1);
   p.fd_L2 = make_fastdiv((uint32_t)plan->geom.L2);
@@ -720,6 +738,9 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
       case Lat_bcc_1_2::id: launch_obs_spec<Lat_bcc_1_2>(p, grid, s); break;
       default: launch_obs_spec<Lat_fcc_1>(p, grid, s); break;
     }
+  } else if (obs_columns(plan, storage)) {
+    const int rc = launch_word_columns(plan, p, s);
+    if (rc != SCK_OK) return rc;
   } else if (p.storage == 2 && obs_words_ok(plan, storage)) {
     observables_words_kernel<<<dim3(p.blocks_per_rep, (p.B + 31) / 32), 256, 0, s>>>(p);
   } else if (p.storage == 2) observables_kernel<1, 2><<<grid, 256, 0, s>>>(p);
@@ -734,8 +755,7 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
 
 int launch_observables_finish(const double* partial, int B, int blocks_per_rep, int b, int n, double* E, double* M,
                               cudaStream_t s) {
-  dim3 fb(OBS_VALUES, 8);
-  observables_finish<<<(B + 7) / 8, fb, 0, s>>>(partial, B, blocks_per_rep, b, n, E, M);
+  observables_finish<<<B, dim3(OBS_VALUES, FINISH_LANES), 0, s>>>(partial, blocks_per_rep, b, n, E, M);
   return cuda_status(cudaGetLastError(), "observables finish");
 }
 
@@ -780,7 +800,7 @@ extern "C" int sck_observables_noalloc(const sck_plan* plan, const sck_buffers* 
     set_error("the system needs its mask / k1 buffers");
     return SCK_ERR_INVALID;
   }
-  const size_t need = (size_t)batch * obs_launch_blocks(plan, storage, batch) * OBS_VALUES;
+  const size_t need = (size_t)batch * obs_scratch_slots(plan, storage, batch) * OBS_VALUES;
   if (need > kScratchDoubles) {
     set_error("no-alloc observables: " + std::to_string(need * sizeof(double)) + " bytes of partial sums exceed the " +
               std::to_string(kScratchDoubles * sizeof(double)) + "-byte scratch; use sck_observables with a workspace");
@@ -789,5 +809,6 @@ extern "C" int sck_observables_noalloc(const sck_plan* plan, const sck_buffers* 
   double* scratch = nullptr;
   const int rc = scratch_address(&scratch);
   if (rc != SCK_OK) return rc;
-  return launch_observables(plan, spins, storage, batch, buf->mask, buf->k1, E, M, scratch, (cudaStream_t)stream);
+  return launch_observables(plan, spins, storage, batch, buf->mask, buf->k1, E, M, scratch, (cudaStream_t)stream,
+                            (int)(kScratchDoubles / ((size_t)batch * OBS_VALUES)));
 }
