@@ -349,6 +349,7 @@ int sck_plan_create(const sck_system_desc* d, int32_t batch, int32_t mode, sck_p
   p->field = (d->n == 1 && d->h64[0] != 0.0) ? 1 : 0;
   p->spec = find_spec(p);
   p->word_spec = find_word_spec(p);
+  p->resident_spec = find_resident_spec(p);
   if (mode == SCK_MODE_QUAD) {
     std::string why;
     if (!quad_ok(p, &why)) {
@@ -392,6 +393,7 @@ int sck_plan_tune(sck_plan* plan, int32_t specialised, int64_t l2_budget_bytes, 
   if (resident_limit_bytes > kResidentMax) return fail(SCK_ERR_INVALID, "resident limit above 220 KiB of shared memory");
   plan->spec = (specialised || plan->mode == SCK_MODE_QUAD) ? find_spec(plan) : 0;   // interleaved: always
   plan->word_spec = specialised ? find_word_spec(plan) : 0;
+  plan->resident_spec = specialised ? find_resident_spec(plan) : 0;
   plan->kernel_kind = specialised >= 3 ? 3 : (specialised >= 2 ? 2 : 1);
   plan->l2_budget = l2_budget_bytes;
   plan->resident_limit = resident_limit_bytes;
@@ -593,7 +595,7 @@ int sck_sweep(const sck_plan* plan, const sck_buffers* buf, int32_t n_sweeps, vo
   }
   if (use_resident(plan)) {
     const Common c = make_common(plan, buf, buf->spins);
-    rc = launch_resident(plan, c, n_sweeps, s);
+    rc = plan->resident_spec ? launch_lattice_resident(plan, c, n_sweeps, s) : launch_resident(plan, c, n_sweeps, s);
     if (rc != SCK_OK) return rc;
     return launch_advance(buf->state, n_sweeps, s);
   }

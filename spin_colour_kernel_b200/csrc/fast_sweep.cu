@@ -15,7 +15,7 @@
 // runs class c on group k - c for every c at once (a diagonal over (group, class)): the C launches that touch a
 // group run back to back, so after its first read from HBM a group stays in L2 until its sweep is done. Each
 // replica's chain is unchanged: its classes still run in order, one launch after another.
-#include "spec_site.cuh"
+#include "words.cuh"
 
 namespace sck {
 
@@ -29,8 +29,7 @@ __global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ 
   const int ti = blockIdx.y / p.units_per_task;
   const int unit = blockIdx.y - ti * p.units_per_task;
   const Task task = p.tasks[ti];
-  constexpr int per_unit = N == 1 ? 1 : 2;
-  const int rep = task.rep_begin + unit * per_unit;
+  const int rep = task.rep_begin + unit * 2;
   if (rep >= task.rep_end) return;
   int x, y, z;
   if (!class_site(p.c, task.colour, task.alpha, t, x, y, z)) return;
@@ -38,11 +37,90 @@ __global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ 
   static_for<0, Lat::b>([&](auto ac) {
     constexpr int a = decltype(ac)::value;
     if (a != task.alpha) return;
-    if constexpr (N == 1) {
-      ising_spec_site<Lat, a, ST, PER>(p.c, rep, x, y, z, key);
-    } else {
-      vec_spec_pair<Lat, a, N, PER, NSL>(p.c, p.J[a], rep, rep + 1 < task.rep_end, x, y, z, key);
-    }
+    vec_spec_pair<Lat, a, N, PER, NSL>(p.c, p.J[a], rep, rep + 1 < task.rep_end, x, y, z, key);
+  });
+}
+
+// One class of int8 or float32 Ising replicas. A thread keeps its class site for several replicas: site, neighbour
+// offsets and, per block, the sweep's round keys are formed once, and two replicas' loads are in flight together.
+// Bound by instruction issue; the Philox call alone (36 instructions, 70 cycles of a scheduler's multiply pipe) is
+// 131 us a sweep of 64^3 x 256 sites. Grid (class sites / 256, replica rows of p.per).
+struct IsingClassParams {
+  Common c;
+  int colour, alpha, per;
+};
+
+template <class Lat, typename ST, bool PER>
+__global__ void __launch_bounds__(256, 4) ising_class_kernel(const __grid_constant__ IsingClassParams p) {
+  __shared__ uint4 keys[5];
+  const Common& c = p.c;
+  const Geometry& g = c.g;
+  if (threadIdx.x < 10) write_keys(keys, sweep_key(c.state), threadIdx.x);
+  __syncthreads();
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  int x, y, z;
+  if (t >= (uint32_t)c.rows * (uint32_t)c.bx || !class_site(c, p.colour, p.alpha, t, x, y, z)) return;
+  const uint32_t own = (uint32_t)(p.alpha * g.plane + (z * g.L2 + y) * g.L1 + x);
+  if (g.has_mask && c.mask[own] == 0) return;
+  const RoundKeys rk = shared_keys(keys);
+  const bool barker = g.acceptance == SCK_BARKER;
+  const Around<Lat::reach, PER> nb(g, x, y, z);
+  static_for<0, Lat::b>([&](auto ac) {
+    constexpr int A = decltype(ac)::value;
+    if (A != p.alpha) return;
+    constexpr int Z = Lat::n_bonds(A);
+    uint32_t off[Z];
+    bool ok[Z];
+    static_for<0, Z>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      constexpr BondC bd = Lat::bond(A, i);
+      off[i] = (uint32_t)nb.index(g, bd);
+      ok[i] = nb.valid(bd);
+    });
+    const int r0 = (int)blockIdx.y * p.per, r1 = r0 + p.per < c.B ? r0 + p.per : c.B;
+    const uint32_t nsite = (uint32_t)g.nsite;
+    const ST* src = (const ST*)c.src + (size_t)r0 * nsite;
+    ST* dst = (ST*)c.dst + (size_t)r0 * nsite;
+    const float* tab = (const float*)c.table + (size_t)r0 * c.lut_rep_stride + A * c.keys;
+    uint32_t ctr = counter_of(r0, g.nsite, (int)own);
+    auto replicas = [&](auto nc) {
+      constexpr int N = decltype(nc)::value;
+      int s[N], v[N][Z];
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        const ST* sr = src + (size_t)r * nsite;
+        s[r] = sgn(sr[own]);
+#pragma unroll
+        for (int i = 0; i < Z; ++i) v[r][i] = ok[i] ? sgn(__ldg(sr + off[i])) : 0;
+      }
+      float e[N];
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        int k = s[r] > 0 ? 1 : 0, stride = 2;
+        static_for<0, Lat::groups>([&](auto gc) {
+          using R = GroupRange<Lat, A, decltype(gc)::value>;
+          int G = 0;
+#pragma unroll
+          for (int i = R::begin; i < R::end; ++i) G += v[r][i];
+          k += (G + (R::end - R::begin)) * stride;
+          stride *= 2 * (R::end - R::begin) + 1;
+        });
+        e[r] = tab[(size_t)r * c.lut_rep_stride + k];
+      }
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        const float u = to_uniform(philox_keys(ctr + (uint32_t)r * nsite, rk).x0);
+        const bool acc = barker ? __fmul_rn(u, __fadd_rn(1.0f, e[r])) < 1.0f : u < e[r];
+        if (acc) dst[(size_t)r * nsite + own] = (ST)(-s[r]);
+      }
+      src += (size_t)N * nsite;
+      dst += (size_t)N * nsite;
+      tab += (size_t)N * c.lut_rep_stride;
+      ctr += (uint32_t)N * nsite;
+    };
+    int r = r0;
+    for (; r + 2 <= r1; r += 2) replicas(std::integral_constant<int, 2>{});
+    if (r < r1) replicas(std::integral_constant<int, 1>{});
   });
 }
 
@@ -156,31 +234,34 @@ int stream_wait_timeouts(unsigned long long* count) {
 
 // ------------------------------------------------------------------------------------------ host: matching
 template <class Lat>
-static bool matches(const sck_plan* p) {
+static bool matches(const sck_plan* p, bool extras) {
   const sck_system_desc& d = p->desc;
   if (d.b != Lat::b || d.dim != Lat::dim) return false;
   for (int a = 0; a < d.b; ++a) {
     const sck_sublattice& s = d.sub[a];
-    if (s.n_groups != Lat::groups || s.n_bonds != Lat::n_bonds(a) || s.n_extra != 0) return false;
+    if (s.n_groups != Lat::groups || s.n_bonds != Lat::n_bonds(a) || (s.n_extra != 0 && !extras))
+      return false;
     for (int gi = 0; gi < s.n_groups; ++gi)
       if (!s.group_apply[gi] || s.group_end[gi] != Lat::group_end(a, gi)) return false;
     for (int i = 0; i < s.n_bonds; ++i) {
       const BondC b = Lat::bond(a, i);
       const sck_bond& e = s.bonds[i];
-      if (e.alpha2 != b.a2 || e.d[0] != b.dx || e.d[1] != b.dy || e.d[2] != b.dz || e.extra != -1) return false;
+      if (e.alpha2 != b.a2 || e.d[0] != b.dx || e.d[1] != b.dy || e.d[2] != b.dz || (e.extra != -1 && !extras))
+        return false;
     }
   }
   return true;
 }
 
-// Id of the compile-time table that equals the plan's bond lists, or 0.
-int match_lattice(const sck_plan* p) {
-  if (matches<Lat_square_1>(p)) return Lat_square_1::id;
-  if (matches<Lat_triangular_1>(p)) return Lat_triangular_1::id;
-  if (matches<Lat_sc_1>(p)) return Lat_sc_1::id;
-  if (matches<Lat_bcc_1>(p)) return Lat_bcc_1::id;
-  if (matches<Lat_bcc_1_2>(p)) return Lat_bcc_1_2::id;
-  if (matches<Lat_fcc_1>(p)) return Lat_fcc_1::id;
+// Id of the compile-time table that equals the plan's bond lists, or 0; with `extras`, extra matrices on its bonds are left
+// aside.
+int match_lattice(const sck_plan* p, bool extras) {
+  if (matches<Lat_square_1>(p, extras)) return Lat_square_1::id;
+  if (matches<Lat_triangular_1>(p, extras)) return Lat_triangular_1::id;
+  if (matches<Lat_sc_1>(p, extras)) return Lat_sc_1::id;
+  if (matches<Lat_bcc_1>(p, extras)) return Lat_bcc_1::id;
+  if (matches<Lat_bcc_1_2>(p, extras)) return Lat_bcc_1_2::id;
+  if (matches<Lat_fcc_1>(p, extras)) return Lat_fcc_1::id;
   return 0;
 }
 
@@ -192,10 +273,10 @@ int find_spec(const sck_plan* p) {
 // ------------------------------------------------------------------------------------------- host: launches
 template <class Lat, int N, typename ST, bool PER, int NSL, class P>
 static void launch_one(const P& p, dim3 grid, cudaStream_t s) {
-  if constexpr (std::is_same_v<P, SpecParams>)
-    spec_task_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
-  else
+  if constexpr (!std::is_same_v<P, SpecParams>)
     stream_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
+  else if constexpr (N > 1)               // Ising class launches: ising_class_kernel
+    spec_task_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
 }
 
 template <class Lat, int N, bool PER, class P>
@@ -268,7 +349,7 @@ static void launch_spec_grid(const sck_plan* plan, const P& p, dim3 grid, cudaSt
   }
 }
 
-static int slot_replicas(const sck_plan* plan) { return plan->geom.n == 1 || seg_kernel_ok(plan) ? 1 : 2; }
+static int slot_replicas(const sck_plan* plan) { return seg_kernel_ok(plan) ? 1 : 2; }
 
 static int launch_tasks(const sck_plan* plan, SpecParams& p, cudaStream_t s) {
   const int per_unit = slot_replicas(plan);
@@ -295,8 +376,44 @@ static SpecParams spec_params(const sck_plan* plan, const Common& c) {
   return p;
 }
 
+template <class Lat>
+static void launch_ising_t(const sck_plan* plan, const IsingClassParams& p, dim3 grid, cudaStream_t s) {
+  const bool per = periodic_box<Lat>(plan);
+  if (plan->mode == SCK_MODE_INT8) {
+    if (per) ising_class_kernel<Lat, int8_t, true><<<grid, 256, 0, s>>>(p);
+    else ising_class_kernel<Lat, int8_t, false><<<grid, 256, 0, s>>>(p);
+  } else {
+    if (per) ising_class_kernel<Lat, float, true><<<grid, 256, 0, s>>>(p);
+    else ising_class_kernel<Lat, float, false><<<grid, 256, 0, s>>>(p);
+  }
+}
+
+// Replicas per thread: up to eight, as long as the launch keeps sixteen blocks per SM (four rounds of its four).
+static int launch_ising_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s) {
+  IsingClassParams p;
+  p.c = c;
+  p.colour = colour;
+  p.alpha = alpha;
+  const uint32_t per = (uint32_t)c.rows * (uint32_t)c.bx;
+  const unsigned bx = (per + 255) / 256;
+  p.per = 1;
+  while (p.per < 8 && (long long)bx * ((c.B + 2 * p.per - 1) / (2 * p.per)) >= 148 * 16) p.per *= 2;
+  if ((c.B + p.per - 1) / p.per > 65535) p.per = (c.B + 65534) / 65535;
+  const dim3 grid(bx, (unsigned)((c.B + p.per - 1) / p.per));
+  switch (plan->spec) {
+    case Lat_square_1::id: launch_ising_t<Lat_square_1>(plan, p, grid, s); break;
+    case Lat_triangular_1::id: launch_ising_t<Lat_triangular_1>(plan, p, grid, s); break;
+    case Lat_sc_1::id: launch_ising_t<Lat_sc_1>(plan, p, grid, s); break;
+    case Lat_bcc_1::id: launch_ising_t<Lat_bcc_1>(plan, p, grid, s); break;
+    case Lat_bcc_1_2::id: launch_ising_t<Lat_bcc_1_2>(plan, p, grid, s); break;
+    default: launch_ising_t<Lat_fcc_1>(plan, p, grid, s); break;
+  }
+  return cuda_status(cudaGetLastError(), "Ising class launch");
+}
+
 // One class over all replicas, in chunks of at most 65535 grid rows.
 int launch_spec_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s) {
+  if (plan->geom.n == 1) return launch_ising_class(plan, c, colour, alpha, s);
   if (tile_kernel_ok(plan)) return launch_tile_class(plan, c, colour, alpha, s);
   SpecParams p = spec_params(plan, c);
   const int chunk = 65535 * slot_replicas(plan);

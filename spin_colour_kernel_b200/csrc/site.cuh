@@ -51,6 +51,63 @@ __device__ __forceinline__ void ising_site(const Common& c, const SubDev& sub, i
 }
 
 // ------------------------------------------------------------------------------------------- vector models
+// Proposal, energy change, acceptance and store of site `own` with spin s and bond field v; the external field is added here.
+template <int N>
+__device__ __forceinline__ void vec_finish(const Common& c, int own, int rep, int32_t key, const float (&s)[N],
+                                           float (&v)[N], const float* src, float* dst) {
+  const Geometry& g = c.g;
+  const int NS = g.nsite;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (c.hnz[k]) v[k] = __fadd_rn(v[k], c.h[k]);
+
+  const Philox4 r = philox4x32_10(counter32(rep, g.nsite, own), 0u, key_lo(key), key_hi(key));
+  const float u0 = to_uniform(r.x0);
+  const float TWO_PI = 6.2831855f;
+  float t[N];
+  if (N == 2) {
+    float sn, cs;
+    sincosf(__fmul_rn(TWO_PI, to_uniform(r.x1)), &sn, &cs);
+    t[0] = cs;
+    t[1 % N] = sn;
+  } else if (N == 3) {
+    const float cz = __fsub_rn(__fmul_rn(2.0f, to_uniform(r.x1)), 1.0f);
+    float sn, cs;
+    sincosf(__fmul_rn(TWO_PI, to_uniform(r.x2)), &sn, &cs);
+    const float rr = sqrtf(fmaxf(__fsub_rn(1.0f, __fmul_rn(cz, cz)), 0.0f));
+    t[0] = __fmul_rn(rr, cs);
+    t[1 % N] = __fmul_rn(rr, sn);
+    t[2 % N] = cz;
+  } else {
+    t[0] = -s[0];
+  }
+  float d = __fmul_rn(__fsub_rn(t[0], s[0]), v[0]);
+#pragma unroll
+  for (int k = 1; k < N; ++k) d = __fadd_rn(d, __fmul_rn(__fsub_rn(t[k], s[k]), v[k]));
+  float dE = -d;
+  if (N == 3 && g.has_cubic) {
+    const float k1 = c.k1[own];
+    auto aniso = [&](const float* p) {
+      const float q01 = __fmul_rn(p[0], p[1 % N]), q02 = __fmul_rn(p[0], p[2 % N]);
+      const float q12 = __fmul_rn(p[1 % N], p[2 % N]);
+      const float tri = __fmul_rn(q01, p[2 % N]);
+      const float quad = __fadd_rn(__fadd_rn(__fmul_rn(q01, q01), __fmul_rn(q02, q02)), __fmul_rn(q12, q12));
+      return __fadd_rn(__fmul_rn(k1, quad), __fmul_rn(__fmul_rn(c.k2, tri), tri));
+    };
+    dE = __fadd_rn(dE, __fsub_rn(aniso(t), aniso(s)));
+  }
+  const float beta = c.beta[rep];
+  bool acc;
+  if (g.acceptance == SCK_BARKER)
+    acc = __fmul_rn(u0, __fadd_rn(1.0f, expf(__fmul_rn(beta, dE)))) < 1.0f;
+  else
+    acc = u0 < expf(__fmul_rn(-beta, dE));
+  if (acc || (const void*)src != (const void*)dst) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) dst[k * NS + own] = acc ? t[k] : s[k];
+  }
+}
+
 template <int N>
 __device__ __forceinline__ void vec_site(const Common& c, const SubDev& sub, int alpha, int rep, int x, int y,
                                          int z, int32_t key, const float* src, float* dst) {
@@ -104,55 +161,7 @@ __device__ __forceinline__ void vec_site(const Common& c, const SubDev& sub, int
       if (any) v[k] = __fadd_rn(v[k], tot);
     }
   }
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-    if (c.hnz[k]) v[k] = __fadd_rn(v[k], c.h[k]);
-
-  const Philox4 r = philox4x32_10(counter32(rep, g.nsite, own), 0u, key_lo(key), key_hi(key));
-  const float u0 = to_uniform(r.x0);
-  const float TWO_PI = 6.2831855f;
-  float t[N];
-  if (N == 2) {
-    float sn, cs;
-    sincosf(__fmul_rn(TWO_PI, to_uniform(r.x1)), &sn, &cs);
-    t[0] = cs;
-    t[1 % N] = sn;
-  } else if (N == 3) {
-    const float cz = __fsub_rn(__fmul_rn(2.0f, to_uniform(r.x1)), 1.0f);
-    float sn, cs;
-    sincosf(__fmul_rn(TWO_PI, to_uniform(r.x2)), &sn, &cs);
-    const float rr = sqrtf(fmaxf(__fsub_rn(1.0f, __fmul_rn(cz, cz)), 0.0f));
-    t[0] = __fmul_rn(rr, cs);
-    t[1 % N] = __fmul_rn(rr, sn);
-    t[2 % N] = cz;
-  } else {
-    t[0] = -s[0];
-  }
-  float d = __fmul_rn(__fsub_rn(t[0], s[0]), v[0]);
-#pragma unroll
-  for (int k = 1; k < N; ++k) d = __fadd_rn(d, __fmul_rn(__fsub_rn(t[k], s[k]), v[k]));
-  float dE = -d;
-  if (N == 3 && g.has_cubic) {
-    const float k1 = c.k1[own];
-    auto aniso = [&](const float* p) {
-      const float q01 = __fmul_rn(p[0], p[1 % N]), q02 = __fmul_rn(p[0], p[2 % N]);
-      const float q12 = __fmul_rn(p[1 % N], p[2 % N]);
-      const float tri = __fmul_rn(q01, p[2 % N]);
-      const float quad = __fadd_rn(__fadd_rn(__fmul_rn(q01, q01), __fmul_rn(q02, q02)), __fmul_rn(q12, q12));
-      return __fadd_rn(__fmul_rn(k1, quad), __fmul_rn(__fmul_rn(c.k2, tri), tri));
-    };
-    dE = __fadd_rn(dE, __fsub_rn(aniso(t), aniso(s)));
-  }
-  const float beta = c.beta[rep];
-  bool acc;
-  if (g.acceptance == SCK_BARKER)
-    acc = __fmul_rn(u0, __fadd_rn(1.0f, expf(__fmul_rn(beta, dE)))) < 1.0f;
-  else
-    acc = u0 < expf(__fmul_rn(-beta, dE));
-  if (acc || (const void*)src != (const void*)dst) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) dst[k * NS + own] = acc ? t[k] : s[k];
-  }
+  vec_finish<N>(c, own, rep, key, s, v, src, dst);
 }
 
 }  // namespace sck

@@ -1,0 +1,75 @@
+"""Resident sweeps on lattice tables (csrc/resident.cu) and the int8 / float32 Ising class kernel (csrc/fast_sweep.cu)
+against the generic kernels, which share their arithmetic: the chains are equal bit for bit. Boxes whose class has
+fewer sites than a block, more than a block, and a remainder; masks, open axes, extra matrices, fields, anisotropy,
+both acceptance rules; more sweeps than a block's keys; replica counts that leave a replica over."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from spin_colour_kernel_b200 import crystals as cr
+from spin_colour_kernel_b200 import system as sy
+from spin_colour_kernel_b200.sampler import Sampler
+
+pytestmark = pytest.mark.gpu
+
+
+def _sys(n, crystal, box, per=None, shells=(1,), J=None, mask=False, **kw):
+    c = cr.make(crystal, shells)
+    m = None
+    if mask:
+        shape = (c.b, box[2] if c.D == 3 else 1, box[1], box[0])
+        m = np.random.default_rng(5).random(shape) < 0.8
+    return sy.System(f"{crystal} n={n}", n, c, box, per or (True,) * c.D, J or {s: 1.0 for s in shells}, mask=m, **kw)
+
+
+RESIDENT = {
+    "nanodot": lambda: sy.nanodot(6.0, 3),
+    "nanodot-large": lambda: sy.nanodot(18.3, 5),
+    "ising-square": lambda: _sys(1, "square", (32, 32)),
+    "ising-sc-open": lambda: _sys(1, "sc", (7, 6, 5), (False,) * 3, mask=True, h=(0.3,), acceptance="barker"),
+    "ising-fcc": lambda: _sys(1, "fcc", (6, 5, 7)),
+    "ising-bcc-j1j2": lambda: _sys(1, "bcc", (8, 6, 4), shells=(1, 2), J={1: 1.0, 2: -0.4}),
+    "xy-triangular": lambda: _sys(2, "triangular", (33, 27), h=(0.1, 0.0)),
+    "heisenberg-bcc": lambda: _sys(3, "bcc", (9, 8, 7), acceptance="barker"),
+    "heisenberg-dmi": lambda: _sys(3, "square", (40, 30), extra={0: np.array([[0, .3, 0], [-.3, 0, .1], [0, -.1, 0]])}),
+}
+
+
+@pytest.mark.parametrize("name", sorted(RESIDENT))
+@pytest.mark.parametrize("f32", [False, True])
+def test_resident_lattice_kernels_equal_the_generic_one(name, f32):
+    s = RESIDENT[name]()
+    if s.n > 1 and not f32:
+        pytest.skip("int8 holds Ising spins")
+    B = 5
+    kw = dict(packed=False, spin_dtype=torch.float32 if f32 else torch.int8) if s.n == 1 else {}
+    A, G = (Sampler(s, B, device="cuda", seed=9, **kw) for _ in range(2))
+    G.tune(False)
+    assert A.path()["resident"] and G.path()["resident"]
+    S = A.init_spins(seed=2)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(0.4, 3.0, B))
+        X.sweep(Y, 35)
+    assert torch.equal(A.state, G.state)
+    assert torch.equal(S, S2)
+
+
+@pytest.mark.parametrize("name", ["ising-square", "ising-sc-open", "ising-fcc", "ising-bcc-j1j2"])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("B", [1, 7, 300])
+def test_ising_class_kernel_equals_the_generic_one(name, f32, B):
+    s = RESIDENT[name]()
+    kw = dict(packed=False, spin_dtype=torch.float32 if f32 else torch.int8)
+    A, G = (Sampler(s, B, device="cuda", seed=3, **kw) for _ in range(2))
+    A.tune(True, 0, 0)
+    G.tune(False, 0, 0)
+    S = A.init_spins(seed=2)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(1.5, 6.0, B))
+        X.sweep(Y, 2)
+    assert torch.equal(S, S2)
