@@ -51,12 +51,12 @@ __device__ __forceinline__ void ising_site(const Common& c, const SubDev& sub, i
 }
 
 // ------------------------------------------------------------------------------------------- vector models
-// Proposal, energy change, acceptance and store of site `own` with spin s and bond field v; the external field is added here.
+// Proposal t, energy change and acceptance of site `own` with spin s and bond field v (the external field is added
+// here).
 template <int N>
-__device__ __forceinline__ void vec_finish(const Common& c, int own, int rep, int32_t key, const float (&s)[N],
-                                           float (&v)[N], const float* src, float* dst) {
+__device__ __forceinline__ bool vec_decide(const Common& c, int own, int rep, int32_t key, const float (&s)[N],
+                                           float (&v)[N], float (&t)[N]) {
   const Geometry& g = c.g;
-  const int NS = g.nsite;
 #pragma unroll
   for (int k = 0; k < N; ++k)
     if (c.hnz[k]) v[k] = __fadd_rn(v[k], c.h[k]);
@@ -64,7 +64,6 @@ __device__ __forceinline__ void vec_finish(const Common& c, int own, int rep, in
   const Philox4 r = philox4x32_10(counter32(rep, g.nsite, own), 0u, key_lo(key), key_hi(key));
   const float u0 = to_uniform(r.x0);
   const float TWO_PI = 6.2831855f;
-  float t[N];
   if (N == 2) {
     float sn, cs;
     sincosf(__fmul_rn(TWO_PI, to_uniform(r.x1)), &sn, &cs);
@@ -97,11 +96,17 @@ __device__ __forceinline__ void vec_finish(const Common& c, int own, int rep, in
     dE = __fadd_rn(dE, __fsub_rn(aniso(t), aniso(s)));
   }
   const float beta = c.beta[rep];
-  bool acc;
-  if (g.acceptance == SCK_BARKER)
-    acc = __fmul_rn(u0, __fadd_rn(1.0f, expf(__fmul_rn(beta, dE)))) < 1.0f;
-  else
-    acc = u0 < expf(__fmul_rn(-beta, dE));
+  if (g.acceptance == SCK_BARKER) return __fmul_rn(u0, __fadd_rn(1.0f, expf(__fmul_rn(beta, dE)))) < 1.0f;
+  return u0 < expf(__fmul_rn(-beta, dE));
+}
+
+// The same with the store: dst gets the spin the site ends with.
+template <int N>
+__device__ __forceinline__ void vec_finish(const Common& c, int own, int rep, int32_t key, const float (&s)[N],
+                                           float (&v)[N], const float* src, float* dst) {
+  float t[N];
+  const bool acc = vec_decide<N>(c, own, rep, key, s, v, t);
+  const int NS = c.g.nsite;
   if (acc || (const void*)src != (const void*)dst) {
 #pragma unroll
     for (int k = 0; k < N; ++k) dst[k * NS + own] = acc ? t[k] : s[k];

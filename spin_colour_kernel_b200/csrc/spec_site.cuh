@@ -21,6 +21,13 @@ struct Around {
     return q;
   }
 
+  // wrap_axis for offsets of at most one cell, which one wrap always brings back into the box
+  __device__ __forceinline__ static int axis1(int x, int d, int L, int periodic) {
+    const int q = x + d;
+    const int w = q < 0 ? L - 1 : (q >= L ? 0 : q);
+    return w == q || periodic ? w : -1;
+  }
+
   __device__ __forceinline__ Around(const Geometry& g, int x, int y, int z) {
 #pragma unroll
     for (int d = -R; d <= R; ++d) {
@@ -30,9 +37,9 @@ struct Around {
         qy = wrap1(y, d, g.L2);
         qz = g.dim == 3 ? wrap1(z, d, g.L3) : z;
       } else {
-        qx = wrap_axis(x, d, g.L1, g.per[0]);
-        qy = wrap_axis(y, d, g.L2, g.per[1]);
-        qz = wrap_axis(z, d, g.L3, g.per[2]);
+        qx = R == 1 ? axis1(x, d, g.L1, g.per[0]) : wrap_axis(x, d, g.L1, g.per[0]);
+        qy = R == 1 ? axis1(y, d, g.L2, g.per[1]) : wrap_axis(y, d, g.L2, g.per[1]);
+        qz = R == 1 ? axis1(z, d, g.L3, g.per[2]) : wrap_axis(z, d, g.L3, g.per[2]);
       }
       xv[d + R] = qx >= 0;
       yv[d + R] = qy >= 0;

@@ -1,7 +1,8 @@
 """Resident sweeps on lattice tables (csrc/resident.cu) and the int8 / float32 Ising class kernel (csrc/fast_sweep.cu)
 against the generic kernels, which share their arithmetic: the chains are equal bit for bit. Boxes whose class has
 fewer sites than a block, more than a block, and a remainder; masks, open axes, extra matrices, fields, anisotropy,
-both acceptance rules; more sweeps than a block's keys; replica counts that leave a replica over."""
+both acceptance rules; calls with and without neighbour lists, a replica shared by two blocks (the large nanodot),
+more sweeps than a block's keys; replica counts that leave a replica over."""
 
 from __future__ import annotations
 
@@ -40,7 +41,8 @@ RESIDENT = {
 
 @pytest.mark.parametrize("name", sorted(RESIDENT))
 @pytest.mark.parametrize("f32", [False, True])
-def test_resident_lattice_kernels_equal_the_generic_one(name, f32):
+@pytest.mark.parametrize("sweeps", [2, 35])
+def test_resident_lattice_kernels_equal_the_generic_one(name, f32, sweeps):
     s = RESIDENT[name]()
     if s.n > 1 and not f32:
         pytest.skip("int8 holds Ising spins")
@@ -53,7 +55,7 @@ def test_resident_lattice_kernels_equal_the_generic_one(name, f32):
     S2 = S.clone()
     for X, Y in ((A, S), (G, S2)):
         X.set_temperature(torch.linspace(0.4, 3.0, B))
-        X.sweep(Y, 35)
+        X.sweep(Y, sweeps)
     assert torch.equal(A.state, G.state)
     assert torch.equal(S, S2)
 
