@@ -21,6 +21,10 @@ struct LatticeResidentParams {
   float E[SCK_MAX_BASIS][SCK_MAX_EXTRA][9];
   int Enz[SCK_MAX_BASIS][SCK_MAX_EXTRA];
   int has_extra;
+  int single;                             // no row of an extra matrix has two non-zero entries: the next three hold
+  uint8_t live[SCK_MAX_BASIS][16];        //   bit k: bond's row k has an entry
+  int at[SCK_MAX_BASIS][16][3];           //   its column's offset among the listed spins (component x slots)
+  float Erow[SCK_MAX_BASIS][16][3];       //   its value
   int n_classes;
   int classes[128][2];
   int n_sweeps;
@@ -182,13 +186,16 @@ __device__ __forceinline__ int block_rank(bool flag, int* warp_sums, int& sum) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) warp_sums[warp] = __popc(m);
   __syncthreads();
-  int before = 0;
-  sum = 0;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-    const int n = warp_sums[i];
-    before += i < warp ? n : 0;
-    sum += n;
+  // every warp scans the block's sums for itself, one per lane
+  const int own = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0;
+  int incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += up;
   }
+  const int before = __shfl_sync(0xFFFFFFFFu, incl - own, warp);
+  sum = __shfl_sync(0xFFFFFFFFu, incl, 31);
   __syncthreads();
   return before + __popc(m & ((1u << lane) - 1u));
 }
@@ -238,7 +245,7 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
     }
   }
   if (threadIdx.x == 0) first[p.n_classes] = base;
-  for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+  for (int i0 = 0; base < n && i0 < n; i0 += blockDim.x) {   // inactive sites
     __syncthreads();
     const int i = i0 + (int)threadIdx.x;
     int sum;
@@ -298,7 +305,12 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
     }
     const int32_t key = keys[sw % kResidentKeys];
     for (int ci = 0; ci < p.n_classes; ++ci) {
-      const int A = p.classes[ci][1], end = first[ci + 1];
+      const int alpha = p.classes[ci][1], end = first[ci + 1];
+      // the sublattice as a constant: its couplings are then constant-bank operands (indexed, every one is a load
+      // through the address unit; 57 of them an update held the nanodisk step at 155 us)
+      static_for<0, Lat::b>([&](auto ac) {
+      constexpr int A = decltype(ac)::value;
+      if (A != alpha) return;
       for (int sl = first[ci] + rank * (int)blockDim.x + (int)threadIdx.x; sl < end; sl += CL * (int)blockDim.x) {
         uint32_t w[4 * W];
 #pragma unroll
@@ -314,7 +326,7 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
           const int s = sgn(S[sl]);
           int k = s > 0 ? 1 : 0, stride = 2;
           static_for<0, Lat::groups>([&](auto gc) {
-            using R = GroupRange<Lat, 0, decltype(gc)::value>;
+            using R = GroupRange<Lat, A, decltype(gc)::value>;
             int G = 0;
 #pragma unroll
             for (int i = R::begin; i < R::end; ++i) G += sgn(S[list_entry(w, i + 1)]);
@@ -339,7 +351,7 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
           }
           static_for<0, Lat::groups>([&](auto gc) {
             constexpr int gi = decltype(gc)::value;
-            using R = GroupRange<Lat, 0, gi>;
+            using R = GroupRange<Lat, A, gi>;
             float gs[N];
 #pragma unroll
             for (int k = 0; k < N; ++k) gs[k] = 0.0f;
@@ -355,7 +367,20 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
 #pragma unroll
             for (int k = 0; k < N; ++k) v[k] = __fadd_rn(v[k], __fmul_rn(p.J[A][gi], gs[k]));
           });
-          if (p.has_extra) add_extras<Z, N>(p, A, t, v);
+          if (p.single) {
+            // DMI and the like: one product a row, its neighbour component read again at a uniform offset (testing
+            // all nine entries of every bond's matrix cost as much as half the update: 53 of 155 us a ladder step)
+#pragma unroll
+            for (int i = 0; i < Z; ++i) {
+              if (!p.live[A][i]) continue;
+              const ST* q = S + list_entry(w, i + 1);
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                if ((p.live[A][i] >> k) & 1) v[k] = __fadd_rn(v[k], __fmul_rn(p.Erow[A][i][k], q[p.at[A][i][k]]));
+            }
+          } else if (p.has_extra) {
+            add_extras<Z, N>(p, A, t, v);
+          }
           if (vec_decide<N>(c, own, rep, key, s, v, x)) {
 #pragma unroll
             for (int k = 0; k < N; ++k) {
@@ -366,6 +391,7 @@ __global__ void __launch_bounds__(1024) list_resident_kernel(const __grid_consta
           }
         }
       }
+      });
       if constexpr (CL > 1) cg::this_cluster().sync();
       else __syncthreads();
     }
@@ -476,6 +502,21 @@ int launch_lattice_resident(const sck_plan* plan, const Common& c, int n_sweeps,
     }
     if (sub.n_extra > 0) p.has_extra = 1;
   }
+  p.single = p.has_extra;
+  for (int a = 0; a < plan->geom.b; ++a)
+    for (int i = 0; i < 16; ++i) {
+      if (p.extra[a][i] < 0) continue;
+      const int e = p.extra[a][i], nz = p.Enz[a][e];
+      for (int k = 0; k < 3; ++k) {
+        const int row = (nz >> (3 * k)) & 7;
+        if (row == 0) continue;
+        if (row != 1 && row != 2 && row != 4) p.single = 0;
+        const int l = row == 1 ? 0 : (row == 2 ? 1 : 2);
+        p.live[a][i] |= (uint8_t)(1 << k);
+        p.at[a][i][k] = l * (plan->geom.nsite + 1);
+        p.Erow[a][i][k] = p.E[a][e][3 * k + l];
+      }
+    }
   p.n_classes = plan->desc.n_classes;
   for (int i = 0; i < p.n_classes; ++i) {
     p.classes[i][0] = plan->desc.classes[i][0];
