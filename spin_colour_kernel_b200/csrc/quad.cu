@@ -147,11 +147,22 @@ static int quad_blocks_x(const sck_plan* plan) {
   return (int)((per + 255) / 256);
 }
 
+// States that do not stay in L2 (126 MB) are prefetched kPrefetchBlocks blocks ahead: about 1.3 us at 77 blocks
+// finished per us, longer than a read from HBM takes. Measured on the 3D Heisenberg bcc J1-J2 model, one sweep of
+// 64^3 x 2 x 1,536 in us: 10,530 without, 9,900 / 9,710 / 9,900 / 9,880 at 40 / 80 / 120 / 200 ahead, 10,160 at 450,
+// 13,600 at 900 (rows fall out of L2 before they are used). 48^3 x 2: 170 MB 65.7 -> 71.2 attempts/ns, 127 MB
+// 62.9 -> 65.9, 85 MB 64.4 -> 64.0.
+constexpr unsigned kPrefetchBlocks = 100;
+constexpr size_t kPrefetchState = (size_t)96 << 20;
+
 static int launch_quad_params(const sck_plan* plan, QuadParams& p, cudaStream_t s) {
   const int Q = plan->Bp / 4;
+  const size_t state = (size_t)plan->Bp * plan->geom.n * plan->geom.nsite * sizeof(float);
   for (int q0 = 0; q0 < Q; q0 += 65535) {
     p.q0 = q0;
     const int nq = Q - q0 < 65535 ? Q - q0 : 65535;
+    const long long blocks = (long long)quad_blocks_x(plan) * nq;
+    p.ahead = state > kPrefetchState && blocks > 2 * kPrefetchBlocks ? kPrefetchBlocks : 0;
     launch_quad_grid(plan, p, dim3((unsigned)quad_blocks_x(plan), (unsigned)nq), s);
     const int rc = cuda_status(cudaGetLastError(), "interleaved class launch");
     if (rc != SCK_OK) return rc;
