@@ -6,7 +6,7 @@
 // resident capacity of the GPU whose blocks take work items in ticket order from a counter:
 //   - resident items (system, replica), for systems whose replica fits shared memory: the block loads the
 //     replica once and runs every class of every sweep of the call on-chip;
-//   - streaming items (sweep, colour step k, system, replica slot, 2,048-site chunk) for the others, found by
+//   - streaming items (sweep, colour step k, system, replica slot, site chunk) for the others, found by
 //     binary searches over per-step item offsets. Before touching spins, a block waits (bounded) until every item of the
 //     class its item follows is done: class k - 1 of the same system and sweep, or the system's last class of the
 //     previous sweep; per-(system, class) completion counters count finished items. That class holds smaller
@@ -34,7 +34,12 @@ __device__ __forceinline__ void batch_site(const Common& c, const SubDev& sub, i
 }
 
 constexpr int kBatchMaxSystems = 256;
-constexpr int kBatchItemPasses = 8;   // a streaming item: 8 x 256 class sites of one replica slot and class
+// A streaming item is 8 x 256 updates of a replica pair (vector models) or replica (Ising): `passes` runs of 256 class
+// sites for 8 / passes pairs or replicas each. Pairs come first, up to four: a thread then forms a site and its
+// neighbours' offsets once for all of them. Two sweeps of 24 XY systems (40 M attempts): one pair and eight passes
+// 603 us, four pairs and two passes 515; smaller items 592 (half), 781 (a quarter), larger 498 (twice, but fewer
+// items than blocks for small batches).
+constexpr int kBatchItemPasses = 8;
 constexpr int kBatchMaxClasses = 32;
 
 struct SysDev {
@@ -43,8 +48,9 @@ struct SysDev {
   int n_classes;
   int classes[kBatchMaxClasses][2];
   int resident;
-  int chunks;          // streaming items of one class and replica slot (kBatchItemPasses x 256 class sites each)
-  int rpi;             // replicas per streaming item: 2 for vector models (a pair in packed float32x2), 1 Ising
+  int chunks;          // streaming items of one class and replica slot (passes x 256 class sites each)
+  int rpi;             // replicas per streaming item: pairs in packed float32x2 for vector models
+  int passes;
   int spec, per;       // compile-time lattice table of the system (0: generic site update), periodic wrap
   float J[SCK_MAX_BASIS][SCK_MAX_GROUPS];
 };
@@ -120,29 +126,32 @@ __device__ __forceinline__ unsigned batch_ld_acquire(const unsigned* a) {
 }
 
 // The site update of a streaming item: the specialised lattice update (the lattice kernels' arithmetic, a
-// replica pair per thread for vector models) for systems on the square, triangular or simple cubic table, else
+// replica pair at a time for vector models) for systems on the square, triangular or simple cubic table, else
 // the generic update of each replica of the slot.
 template <class Lat, int N, typename ST>
-__device__ __forceinline__ void batch_spec_site(const SysDev& d, int rep0, int x, int y, int z, int32_t key) {
+__device__ __forceinline__ void batch_spec_site(const SysDev& d, int rep0, int rep1, int x, int y, int z, int32_t key) {
   auto run = [&](auto per_c) {
     constexpr bool PER = decltype(per_c)::value;
-    if constexpr (N == 1)
-      ising_spec_site<Lat, 0, ST, PER>(d.c, rep0, x, y, z, key);
-    else
-      vec_spec_pair<Lat, 0, N, PER, 0>(d.c, d.J[0], rep0, rep0 + 1 < d.c.B, x, y, z, key);
+#pragma unroll 1
+    for (int r = rep0; r < rep1; r += N == 1 ? 1 : 2) {
+      if constexpr (N == 1)
+        ising_spec_site<Lat, 0, ST, PER>(d.c, r, x, y, z, key);
+      else
+        vec_spec_pair<Lat, 0, N, PER, 0>(d.c, d.J[0], r, r + 1 < rep1, x, y, z, key);
+    }
   };
   if (d.per) run(std::true_type{});
   else run(std::false_type{});
 }
 
 template <int N, typename ST>
-__device__ __forceinline__ void batch_stream_site(const SysDev& d, int alpha, int rep0, int x, int y, int z,
-                                                  int32_t key) {
-  if (d.spec == Lat_square_1::id) return batch_spec_site<Lat_square_1, N, ST>(d, rep0, x, y, z, key);
-  if (d.spec == Lat_triangular_1::id) return batch_spec_site<Lat_triangular_1, N, ST>(d, rep0, x, y, z, key);
-  if (d.spec == Lat_sc_1::id) return batch_spec_site<Lat_sc_1, N, ST>(d, rep0, x, y, z, key);
+__device__ __forceinline__ void batch_stream_site(const SysDev& d, int alpha, int rep0, int rep1, int x, int y,
+                                                  int z, int32_t key) {
+  if (d.spec == Lat_square_1::id) return batch_spec_site<Lat_square_1, N, ST>(d, rep0, rep1, x, y, z, key);
+  if (d.spec == Lat_triangular_1::id) return batch_spec_site<Lat_triangular_1, N, ST>(d, rep0, rep1, x, y, z, key);
+  if (d.spec == Lat_sc_1::id) return batch_spec_site<Lat_sc_1, N, ST>(d, rep0, rep1, x, y, z, key);
   ST* base = (ST*)d.c.dst;
-  for (int r = rep0; r < rep0 + d.rpi && r < d.c.B; ++r)
+  for (int r = rep0; r < rep1; ++r)
     batch_site<N, ST>(d.c, d.sub[alpha], alpha, r, x, y, z, key, base + (size_t)r * N * d.c.g.nsite);
 }
 
@@ -233,16 +242,18 @@ __global__ void __launch_bounds__(256, 4) batch_persistent_kernel(const BatchDev
       for (int i = threadIdx.x; i < n; i += blockDim.x) home[i] = S[i];
     } else {
       if (kind == 2) {
-        const uint32_t per = (uint32_t)d.c.rows * (uint32_t)d.c.bx;
-        const int colour = d.classes[it.k][0], alpha = d.classes[it.k][1];
-        const int32_t key = sweep_key_at(d.c.state, p.sweep_base + it.sw);
-        const int rep0 = it.rep * d.rpi;
+        const Common& c = d.c;
+        const uint32_t per = (uint32_t)c.rows * (uint32_t)c.bx;
+        const int colour = d.classes[it.k][0], alpha = d.classes[it.k][1], passes = d.passes;
+        const int32_t key = sweep_key_at(c.state, p.sweep_base + it.sw);
+        const int rep0 = it.rep * d.rpi, rep1 = rep0 + d.rpi < c.B ? rep0 + d.rpi : c.B;
+        const uint32_t t0 = (uint32_t)it.chunk * passes * 256u + threadIdx.x;
 #pragma unroll 1
-        for (int pass = 0; pass < kBatchItemPasses; ++pass) {
-          const uint32_t t = ((uint32_t)it.chunk * kBatchItemPasses + pass) * 256u + threadIdx.x;
+        for (int pass = 0; pass < passes; ++pass) {
+          const uint32_t t = t0 + pass * 256u;
           int x, y, z;
-          if (t < per && class_site(d.c, colour, alpha, t, x, y, z))
-            batch_stream_site<N, ST>(d, alpha, rep0, x, y, z, key);
+          if (t < per && class_site(c, colour, alpha, t, x, y, z))
+            batch_stream_site<N, ST>(d, alpha, rep0, rep1, x, y, z, key);
         }
       }
       __syncthreads();
@@ -458,8 +469,12 @@ int sck_batch_bind(sck_batch* b, const sck_buffers* buffers, void* workspace, vo
     }
     d.resident = b->resident[s];
     const long long per = (long long)d.c.rows * d.c.bx;
-    d.chunks = (int)((per + 256 * kBatchItemPasses - 1) / (256 * kBatchItemPasses));
-    d.rpi = plan->geom.n == 1 ? 1 : 2;
+    const int unit = plan->geom.n == 1 ? 1 : 2;
+    int groups = 1;
+    while (groups < 4 && 2 * groups * unit <= plan->Bp) groups *= 2;
+    d.rpi = groups * unit;
+    d.passes = kBatchItemPasses / groups;
+    d.chunks = (int)((per + 256 * d.passes - 1) / (256 * d.passes));
     const bool table = plan->spec == Lat_square_1::id || plan->spec == Lat_triangular_1::id ||
                        plan->spec == Lat_sc_1::id;
     d.spec = table ? plan->spec : 0;

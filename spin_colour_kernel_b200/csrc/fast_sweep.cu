@@ -20,7 +20,9 @@
 namespace sck {
 
 // ------------------------------------------------------------------------------------------------- kernels
-// Grid (ceil(rows * bx / 256), n_tasks * units_per_task). Block y-slot -> (task, replica or replica pair).
+// Grid (ceil(rows * bx / 256), n_tasks * units_per_task). Block y-slot -> (task, `pairs` replica pairs): a thread forms
+// its class site, its neighbours' offsets and the sweep's key once for all of them. Bound by instruction issue (304
+// instructions per attempt with one pair a thread, 75 % of the issue slots, on Heisenberg bcc 32^3 x 2).
 template <class Lat, int N, typename ST, bool PER, int NSL>
 __global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ SpecParams p) {
   const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
@@ -29,15 +31,18 @@ __global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ 
   const int ti = blockIdx.y / p.units_per_task;
   const int unit = blockIdx.y - ti * p.units_per_task;
   const Task task = p.tasks[ti];
-  const int rep = task.rep_begin + unit * 2;
-  if (rep >= task.rep_end) return;
+  const int rep0 = task.rep_begin + unit * 2 * p.pairs;
+  const int rep1 = rep0 + 2 * p.pairs < task.rep_end ? rep0 + 2 * p.pairs : task.rep_end;
+  if (rep0 >= rep1) return;
   int x, y, z;
   if (!class_site(p.c, task.colour, task.alpha, t, x, y, z)) return;
   const int32_t key = sweep_key_at(p.c.state, task.sweep_offset);
   static_for<0, Lat::b>([&](auto ac) {
     constexpr int a = decltype(ac)::value;
     if (a != task.alpha) return;
-    vec_spec_pair<Lat, a, N, PER, NSL>(p.c, p.J[a], rep, rep + 1 < task.rep_end, x, y, z, key);
+#pragma unroll 1
+    for (int rep = rep0; rep < rep1; rep += 2)
+      vec_spec_pair<Lat, a, N, PER, NSL>(p.c, p.J[a], rep, rep + 1 < rep1, x, y, z, key);
   });
 }
 
@@ -352,17 +357,24 @@ static void launch_spec_grid(const sck_plan* plan, const P& p, dim3 grid, cudaSt
 static int slot_replicas(const sck_plan* plan) { return seg_kernel_ok(plan) ? 1 : 2; }
 
 static int launch_tasks(const sck_plan* plan, SpecParams& p, cudaStream_t s) {
-  const int per_unit = slot_replicas(plan);
+  int per_unit = slot_replicas(plan);
   int most = 1;
   for (int i = 0; i < p.n_tasks; ++i) {
     const int n = p.tasks[i].rep_end - p.tasks[i].rep_begin;
     if (n > most) most = n;
   }
+  const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
+  p.pairs = 1;
+  // up to four pairs a thread while eight blocks per SM are left: attempts/ns at one / two / four pairs, Heisenberg bcc
+  // J1-J2 64^3 x 2 x 64: 54 / 60 / 62; XY square 512^2 x 33: 108 / 127 / 144; Heisenberg sc 40^3 x 100: 75 / 79 / 84
+  if (per_unit == 2)
+    while (p.pairs < 4 && (long long)((per + 255) / 256) * p.n_tasks * ((most + 4 * p.pairs - 1) / (4 * p.pairs)) >= 148 * 8)
+      p.pairs *= 2;
+  per_unit *= p.pairs;
   p.units_per_task = (most + per_unit - 1) / per_unit;
   const long long ys = (long long)p.units_per_task * p.n_tasks;
   if (ys > 65535) return cuda_status(cudaErrorInvalidConfiguration, "task launch: too many replicas per launch");
   if (seg_kernel_ok(plan)) return launch_seg_tasks(plan, p, (int)ys, s);
-  const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
   launch_spec_grid(plan, p, dim3((per + 255) / 256, (unsigned)ys), s);
   return cuda_status(cudaGetLastError(), "specialised class launch");
 }

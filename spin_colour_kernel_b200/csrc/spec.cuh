@@ -21,6 +21,7 @@ struct SpecParams {
   float J[SCK_MAX_BASIS][SCK_MAX_GROUPS];
   int n_tasks;
   int units_per_task;     // grid.y slots per task (replicas, or replica pairs for vector models)
+  int pairs;              // lattice kernels: replica pairs a thread updates
   FastDiv fd_segs;        // segment kernels: 4-site segments per row
   Task tasks[kMaxTasks];
 };
