@@ -547,7 +547,7 @@ static int class_launch(const sck_plan* plan, const sck_buffers* buf, const void
   if (plan->mode == SCK_MODE_QUAD) {
     if (src != buf->spins || colour < 0)
       return fail(SCK_ERR_UNSUPPORTED, "interleaved storage updates in place (src = spins, no synchronous control)");
-    return launch_quad_class(plan, buf, colour, alpha, s);
+    return launch_quad_class(plan, buf, colour, alpha, 0, s);
   }
   Common c = make_common(plan, buf, src);
   if (plan->word_spec && colour >= 0 && src == buf->spins) return launch_word_class(plan, c, colour, alpha, s);
@@ -583,15 +583,12 @@ int sck_sweep(const sck_plan* plan, const sck_buffers* buf, int32_t n_sweeps, vo
       if (rc != SCK_OK) return rc;
       return launch_advance(buf->state, n_sweeps, s);
     }
-    for (int k = 0; k < n_sweeps; ++k) {
+    for (int k = 0; k < n_sweeps; ++k)
       for (int i = 0; i < plan->desc.n_classes; ++i) {
-        rc = launch_quad_class(plan, buf, plan->desc.classes[i][0], plan->desc.classes[i][1], s);
+        rc = launch_quad_class(plan, buf, plan->desc.classes[i][0], plan->desc.classes[i][1], k, s);
         if (rc != SCK_OK) return rc;
       }
-      rc = launch_advance(buf->state, 1, s);
-      if (rc != SCK_OK) return rc;
-    }
-    return SCK_OK;
+    return launch_advance(buf->state, n_sweeps, s);
   }
   if (use_resident(plan)) {
     const Common c = make_common(plan, buf, buf->spins);
@@ -612,15 +609,30 @@ int sck_sweep(const sck_plan* plan, const sck_buffers* buf, int32_t n_sweeps, vo
       if (rc != SCK_OK) return rc;
       return launch_advance(buf->state, n_sweeps, s);
     }
+    // the tile kernels read the sweep's key from the state itself
+    const bool once = !tile_kernel_ok(plan);
+    Common ck = c;
     for (int k = 0; k < n_sweeps; ++k) {
+      ck.sweep_offset = once ? k : 0;
       for (int i = 0; i < plan->desc.n_classes; ++i) {
-        rc = launch_spec_class(plan, c, plan->desc.classes[i][0], plan->desc.classes[i][1], s);
+        rc = launch_spec_class(plan, ck, plan->desc.classes[i][0], plan->desc.classes[i][1], s);
         if (rc != SCK_OK) return rc;
       }
-      rc = launch_advance(buf->state, 1, s);
+      if (!once) rc = launch_advance(buf->state, 1, s);
       if (rc != SCK_OK) return rc;
     }
-    return SCK_OK;
+    return once ? launch_advance(buf->state, n_sweeps, s) : SCK_OK;
+  }
+  if (plan->word_spec) {
+    Common c = make_common(plan, buf, buf->spins);
+    for (int k = 0; k < n_sweeps; ++k) {
+      c.sweep_offset = k;
+      for (int i = 0; i < plan->desc.n_classes; ++i) {
+        rc = launch_word_class(plan, c, plan->desc.classes[i][0], plan->desc.classes[i][1], s);
+        if (rc != SCK_OK) return rc;
+      }
+    }
+    return launch_advance(buf->state, n_sweeps, s);
   }
   for (int k = 0; k < n_sweeps; ++k) {
     for (int i = 0; i < plan->desc.n_classes; ++i) {

@@ -73,6 +73,17 @@ __host__ __device__ __forceinline__ uint32_t fdiv(uint32_t n, FastDiv f) {
   return (uint32_t)(((unsigned long long)n * f.m) >> f.s);
 }
 
+// ---------------------------------------------------------------------------------------- dependent launches
+// Class launches of a sweep follow one another on a stream, each reading what the one before wrote. Launched with
+// launch_dependent (internal.h), a kernel's blocks may take their places while the last blocks of the one before
+// still run: every thread of such a kernel calls follow_previous before its first access to memory, which waits for
+// the previous grid to finish with its writes visible, and lets the next one take its place. Loads after it are plain
+// (the compiler may move read-only loads across the wait).
+__device__ __forceinline__ void follow_previous() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------------------------------------------- helpers
 __host__ __device__ inline int colour_of(const Colouring& c, int a, int x, int y, int z) {
   int idx = 0;

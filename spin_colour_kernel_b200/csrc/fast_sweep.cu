@@ -25,6 +25,7 @@ namespace sck {
 // instructions per attempt with one pair a thread, 75 % of the issue slots, on Heisenberg bcc 32^3 x 2).
 template <class Lat, int N, typename ST, bool PER, int NSL>
 __global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ SpecParams p) {
+  follow_previous();
   const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= per) return;
@@ -60,7 +61,8 @@ __global__ void __launch_bounds__(256, 4) ising_class_kernel(const __grid_consta
   __shared__ uint4 keys[5];
   const Common& c = p.c;
   const Geometry& g = c.g;
-  if (threadIdx.x < 10) write_keys(keys, sweep_key(c.state), threadIdx.x);
+  follow_previous();
+  if (threadIdx.x < 10) write_keys(keys, sweep_key_at(c.state, c.sweep_offset), threadIdx.x);
   __syncthreads();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   int x, y, z;
@@ -127,6 +129,82 @@ __global__ void __launch_bounds__(256, 4) ising_class_kernel(const __grid_consta
     for (; r + 2 <= r1; r += 2) replicas(std::integral_constant<int, 2>{});
     if (r < r1) replicas(std::integral_constant<int, 1>{});
   });
+}
+
+// The same for int8 spins on the square and simple cubic lattices, two colours, periodic, rows of whole 4-byte words:
+// a thread takes one word of a row (two class sites) and walks along the last axis. Spins become codes 1 + sign, four
+// at a time, and the codes of the neighbours add up byte by byte; a word's codes serve its own step and its
+// neighbours' along the walk, so a step converts three words and loads three words and a byte for two attempts (the
+// kernel above loads and converts seven bytes for each). What is left is mostly the Philox call. Grid (words of a
+// plane or row / 256, chunks of the walk, replicas).
+struct IsingMarchParams {
+  Common c;
+  int colour, chunk, r0;
+};
+
+// 1 + sign of four int8 spins.
+__device__ __forceinline__ uint32_t spin_codes(uint32_t v) {
+  const uint32_t nonneg = ~v & 0x80808080u;
+  const uint32_t pos = nonneg & ((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu);
+  return (nonneg >> 7) + (pos >> 7);
+}
+
+template <bool CUBIC, bool BARKER>
+__global__ void __launch_bounds__(256, 4) ising_march_kernel(const __grid_constant__ IsingMarchParams p) {
+  constexpr int Z = CUBIC ? 6 : 4;
+  __shared__ uint4 keys[5];
+  __shared__ float tab[2 * (2 * Z + 1)];
+  const Common& c = p.c;
+  const Geometry& g = c.g;
+  follow_previous();
+  const int rep = p.r0 + (int)blockIdx.z;
+  if (threadIdx.x < 10) write_keys(keys, sweep_key_at(c.state, c.sweep_offset), threadIdx.x);
+  for (int i = threadIdx.x; i < 2 * (2 * Z + 1); i += blockDim.x) {
+    const float e = ((const float*)c.table)[(size_t)rep * c.lut_rep_stride + i];
+    tab[i] = BARKER ? __fadd_rn(1.0f, e) : e;
+  }
+  __syncthreads();
+  const int words = g.L1 >> 2;                       // of a row
+  const int col = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (col >= words * (CUBIC ? g.L2 : 1)) return;
+  const int y = CUBIC ? col / words : 0, xw = col - y * words;
+  const int step = CUBIC ? g.L1 * g.L2 : g.L1, len = CUBIC ? g.L3 : g.L2;
+  const int z0 = (int)blockIdx.y * p.chunk, z1 = min(len, z0 + p.chunk);
+  const RoundKeys rk = shared_keys(keys);
+  const int8_t* src = (const int8_t*)c.src + (size_t)rep * g.nsite;
+  int8_t* dst = (int8_t*)c.dst + (size_t)rep * g.nsite;
+  const int row = y * g.L1 + 4 * xw;                 // this word, and those beside it, within a plane
+  const int ym = (y > 0 ? y - 1 : g.L2 - 1) * g.L1 + 4 * xw, yp = (y + 1 < g.L2 ? y + 1 : 0) * g.L1 + 4 * xw;
+  const int left = y * g.L1 + (xw > 0 ? 4 * xw : g.L1) - 1, right = y * g.L1 + (xw + 1 < words ? 4 * xw + 4 : 0);
+  auto word = [&](int at) { return __ldg(reinterpret_cast<const uint32_t*>(src + at)); };
+  // parity of the class in this row: it alternates along the walk
+  int ph = CUBIC ? first_class_x(c, p.colour, 0, y, z0) : first_class_x(c, p.colour, 0, z0, 0);
+  uint32_t below = spin_codes(word((z0 > 0 ? z0 - 1 : len - 1) * step + row)), here = spin_codes(word(z0 * step + row));
+  const uint32_t ctr0 = counter_of(rep, g.nsite, row);
+#pragma unroll 2
+  for (int z = z0; z < z1; ++z) {
+    const int at = z * step;
+    const uint32_t above = spin_codes(word((z + 1 < len ? z + 1 : 0) * step + row));
+    uint32_t sum = below + above;
+    if constexpr (CUBIC) sum += spin_codes(word(at + ym)) + spin_codes(word(at + yp));
+    const uint32_t edge = (uint32_t)(1 + sgn(__ldg(src + at + (ph ? right : left))));
+    const uint32_t even = here & 0x00FF00FFu, odd = (here >> 8) & 0x00FF00FFu;
+    const uint32_t own = ph ? odd : even, other = ph ? even : odd;
+    // neighbours along the row: the other residue's two, and one of them or the edge on the far side
+    const uint32_t side = other + (ph ? (even >> 16) | (edge << 16) : (odd << 16) | edge);
+    const uint32_t key2 = 2u * (((sum >> (8 * ph)) & 0x00FF00FFu) + side) + ((own >> 1) & 0x00010001u);
+    const uint32_t ctr = ctr0 + (uint32_t)(at + ph);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float e = tab[j ? key2 >> 16 : key2 & 0xFFFFu];
+      const float u = to_uniform(philox_keys(ctr + 2u * j, rk).x0);
+      const bool acc = BARKER ? __fmul_rn(u, e) < 1.0f : u < e;
+      if (acc) dst[at + row + ph + 2 * j] = (int8_t)(1 - (int)((own >> (16 * j)) & 0xFFu));
+    }
+    below = here;
+    here = above;
+    ph ^= 1;
+  }
 }
 
 // ----------------------------------------------------------------------------------- the streamed pipeline
@@ -281,7 +359,7 @@ static void launch_one(const P& p, dim3 grid, cudaStream_t s) {
   if constexpr (!std::is_same_v<P, SpecParams>)
     stream_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
   else if constexpr (N > 1)               // Ising class launches: ising_class_kernel
-    spec_task_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
+    launch_dependent(spec_task_kernel<Lat, N, ST, PER, NSL>, grid, 256, s, p);
 }
 
 template <class Lat, int N, bool PER, class P>
@@ -400,6 +478,48 @@ static void launch_ising_t(const sck_plan* plan, const IsingClassParams& p, dim3
   }
 }
 
+// The marching kernel's systems: the walk and both row directions alternate between the two colours; its 4-byte loads
+// need spins that start on 4 bytes.
+static bool ising_march_ok(const sck_plan* plan, const void* spins, int colour) {
+  const Geometry& g = plan->geom;
+  if (colour > 1 || ((uintptr_t)spins & 3u) != 0) return false;
+  if (plan->mode != SCK_MODE_INT8 || g.has_mask || g.L1 % 4 != 0 || !spec_periodic_box(plan)) return false;
+  if (plan->spec != Lat_square_1::id && plan->spec != Lat_sc_1::id) return false;
+  const Colouring& col = plan->col;
+  if (col.r != 1 || col.m[0] != 2) return false;
+  for (int k = 0; k < g.dim; ++k)
+    if (col.K[0][k] != 1) return false;
+  return true;
+}
+
+// Chunks of the walk: long ones convert fewer words twice, short ones keep 16 blocks per SM; at least 8 sites.
+static int launch_ising_march(const sck_plan* plan, const Common& c, int colour, cudaStream_t s) {
+  const Geometry& g = plan->geom;
+  const bool cubic = g.dim == 3, barker = g.acceptance == SCK_BARKER;
+  IsingMarchParams p;
+  p.c = c;
+  p.colour = colour;
+  const int cols = g.L1 / 4 * (cubic ? g.L2 : 1), len = cubic ? g.L3 : g.L2;
+  const long long blocks = (long long)((cols + 255) / 256) * c.B;
+  const long long split = (148 * 16 + blocks - 1) / blocks;
+  p.chunk = (int)((len + split - 1) / split);
+  if (p.chunk < 8) p.chunk = 8;
+  for (p.r0 = 0; p.r0 < c.B; p.r0 += 65535) {
+    const int n = c.B - p.r0 < 65535 ? c.B - p.r0 : 65535;
+    const dim3 grid((unsigned)((cols + 255) / 256), (unsigned)((len + p.chunk - 1) / p.chunk), (unsigned)n);
+    if (cubic) {
+      if (barker) ising_march_kernel<true, true><<<grid, 256, 0, s>>>(p);
+      else ising_march_kernel<true, false><<<grid, 256, 0, s>>>(p);
+    } else {
+      if (barker) ising_march_kernel<false, true><<<grid, 256, 0, s>>>(p);
+      else ising_march_kernel<false, false><<<grid, 256, 0, s>>>(p);
+    }
+    const int rc = cuda_status(cudaGetLastError(), "Ising class launch");
+    if (rc != SCK_OK) return rc;
+  }
+  return SCK_OK;
+}
+
 // Replicas per thread: up to eight, as long as the launch keeps sixteen blocks per SM (four rounds of its four).
 static int launch_ising_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s) {
   IsingClassParams p;
@@ -425,13 +545,14 @@ static int launch_ising_class(const sck_plan* plan, const Common& c, int colour,
 
 // One class over all replicas, in chunks of at most 65535 grid rows.
 int launch_spec_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s) {
-  if (plan->geom.n == 1) return launch_ising_class(plan, c, colour, alpha, s);
+  if (plan->geom.n == 1)
+    return ising_march_ok(plan, c.src, colour) ? launch_ising_march(plan, c, colour, s) : launch_ising_class(plan, c, colour, alpha, s);
   if (tile_kernel_ok(plan)) return launch_tile_class(plan, c, colour, alpha, s);
   SpecParams p = spec_params(plan, c);
   const int chunk = 65535 * slot_replicas(plan);
   for (int r0 = 0; r0 < c.B; r0 += chunk) {
     p.n_tasks = 1;
-    p.tasks[0] = Task{colour, alpha, r0, r0 + chunk < c.B ? r0 + chunk : c.B, 0};
+    p.tasks[0] = Task{colour, alpha, r0, r0 + chunk < c.B ? r0 + chunk : c.B, c.sweep_offset};
     const int rc = launch_tasks(plan, p, s);
     if (rc != SCK_OK) return rc;
   }

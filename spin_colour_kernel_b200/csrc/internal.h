@@ -30,6 +30,7 @@ struct Common {
   const float* beta;
   const void* table;
   const int64_t* state;
+  int sweep_offset;  // the launch's sweep is state[1] + sweep_offset (state advances once per call)
   int* giveup;       // the plan's host-mapped flag, raised (system scope) when a bounded wait gives up; may be null
   unsigned wait_limit;  // polls of a bounded wait before it gives up
   FastDiv fd_bx, fd_L1, fd_L2, fd_m[SCK_MAX_FACTORS];
@@ -151,6 +152,22 @@ void set_error(const std::string& msg);
 int cuda_status(cudaError_t e, const char* where);
 
 // launchers (return SCK_OK or an error code)
+
+// A launch that may overlap the end of the stream's previous kernel; `kernel` calls follow_previous (common.cuh).
+template <class P>
+inline cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, unsigned threads, cudaStream_t s, const P& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 int launch_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s);
 int launch_sequential(const sck_plan* plan, const Common& c, cudaStream_t s);
 int launch_bitwise_class(const sck_plan* plan, const Common& c, int colour, int alpha, cudaStream_t s);
@@ -191,7 +208,8 @@ size_t stream_counter_bytes(const sck_plan* plan, int group);
 int stream_wait_timeouts(unsigned long long* count);   // group pipeline waits that gave up
 // interleaved storage of vector models (quad.cu)
 bool quad_ok(const sck_plan* plan, std::string* why);
-int launch_quad_class(const sck_plan* plan, const sck_buffers* buf, int colour, int alpha, cudaStream_t s);
+int launch_quad_class(const sck_plan* plan, const sck_buffers* buf, int colour, int alpha, int sweep_offset,
+                      cudaStream_t s);
 int launch_quad_convert(const sck_plan* plan, float* flat, float4* quads, int to_flat, cudaStream_t s);
 int quad_obs_blocks(const sck_plan* plan);
 bool quad_measure_fused(const sck_plan* plan);

@@ -170,9 +170,11 @@ static int launch_quad_params(const sck_plan* plan, QuadParams& p, cudaStream_t 
   return SCK_OK;
 }
 
-// One class of every quad (sweep offset 0: the sweep state[1] names).
-int launch_quad_class(const sck_plan* plan, const sck_buffers* buf, int colour, int alpha, cudaStream_t s) {
+// One class of every quad, in sweep state[1] + sweep_offset.
+int launch_quad_class(const sck_plan* plan, const sck_buffers* buf, int colour, int alpha, int sweep_offset,
+                      cudaStream_t s) {
   QuadParams p = quad_params(plan, buf, colour, alpha);
+  p.sweep_offset = sweep_offset;
   return launch_quad_params(plan, p, s);
 }
 

@@ -255,7 +255,15 @@ __global__ void unpack_kernel(const int32_t* __restrict__ words, const int8_t* _
   }
 }
 
-__global__ void advance_kernel(int64_t* state, int n) { state[1] += n; }
+struct AdvanceParams {
+  int64_t* state;
+  int n;
+};
+
+__global__ void advance_kernel(const AdvanceParams p) {
+  follow_previous();
+  p.state[1] += p.n;
+}
 
 // -------------------------------------------------------------------------------------------------- launch
 static dim3 grid2(uint32_t per_unit, int per_block, int units) {
@@ -342,8 +350,7 @@ int launch_unpack(const sck_plan* plan, const int32_t* words, const int8_t* mask
 }
 
 int launch_advance(int64_t* state, int n, cudaStream_t s) {
-  advance_kernel<<<1, 1, 0, s>>>(state, n);
-  return cuda_status(cudaGetLastError(), "advance");
+  return cuda_status(launch_dependent(advance_kernel, dim3(1), 1, s, AdvanceParams{state, n}), "advance");
 }
 
 }  // namespace sck

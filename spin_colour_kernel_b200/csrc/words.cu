@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(256, 5) bitwise_shared_lattice_kernel(const __
   const int u0 = p.u0 + (int)blockIdx.y * p.per_block;
   const int u1 = u0 + p.per_block < units ? u0 + p.per_block : units;
   float* thr = reinterpret_cast<float*>(thr4);
-  if (threadIdx.x < 10) write_keys(keys, sweep_key(c.state), threadIdx.x);
+  follow_previous();
+  if (threadIdx.x < 10) write_keys(keys, sweep_key_at(c.state, c.sweep_offset), threadIdx.x);
   if (threadIdx.x == 32) upper = FIELD ? 0u : 0xFFFFFFFFu;
   __syncthreads();
   for (int i = threadIdx.x; i < 4 * p.per_block * F * (Z + 1); i += blockDim.x) {
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(256, 5) bitwise_shared_lattice_kernel(const __
           const uint32_t* pw = plane + (size_t)(q0 + q) * nsite;
           s0[q] = pw[own];
 #pragma unroll
-          for (int i = 0; i < Z; ++i) x[q][i] = __ldg(pw + off[i]);
+          for (int i = 0; i < Z; ++i) x[q][i] = pw[off[i]];
         }
 #pragma unroll
         for (int q = 0; q < BATCH; ++q) word(q0 + q, s0[q], x[q]);
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(256, 5) bitwise_shared_lattice_kernel(const __
           const uint32_t* pw = plane + (size_t)q * nsite;
           uint32_t x[Z];
 #pragma unroll
-          for (int i = 0; i < Z; ++i) x[i] = __ldg(pw + off[i]);
+          for (int i = 0; i < Z; ++i) x[i] = pw[off[i]];
           word(q, pw[own], x);
         }
     }
@@ -154,9 +155,10 @@ __global__ void __launch_bounds__(256, 4) bitwise_independent_lattice_kernel(con
   __shared__ uint4 keys[8][5];   // round keys of the eight bit groups
   const Common& c = p.c;
   uint32_t* mask = reinterpret_cast<uint32_t*>(mask4);
+  follow_previous();
   if (threadIdx.x < 80) {
     const int grp = threadIdx.x / 10;
-    const long long kg = (long long)sweep_key(c.state) + (long long)(grp + 1) * 104729LL;
+    const long long kg = (long long)sweep_key_at(c.state, c.sweep_offset) + (long long)(grp + 1) * 104729LL;
     write_keys(keys[grp], (int32_t)(kg % 2147483629LL), threadIdx.x % 10);
   }
   uint32_t own = 0, off[Z];
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(256, 4) bitwise_independent_lattice_kernel(con
     const uint32_t s0 = plane[own];
     uint32_t x[Z], cp[NP];
 #pragma unroll
-    for (int i = 0; i < Z; ++i) x[i] = __ldg(plane + off[i]);
+    for (int i = 0; i < Z; ++i) x[i] = plane[off[i]];
     differ_counts<Z>(s0, x, cp);
     auto lanes = [&](int b) {
       uint32_t m[Z + 1];
@@ -225,7 +227,8 @@ __global__ void __launch_bounds__(256, 4) packed_lattice_kernel(const __grid_con
   const Common& c = p.c;
   const int unit = p.u0 + (int)blockIdx.y, w = unit / PARTS, part = unit % PARTS;
   __shared__ uint4 keys[5];
-  if (threadIdx.x < 10) write_keys(keys, sweep_key(c.state), threadIdx.x);
+  follow_previous();
+  if (threadIdx.x < 10) write_keys(keys, sweep_key_at(c.state, c.sweep_offset), threadIdx.x);
   for (int i = threadIdx.x; i < LANES * 2 * (Z + 1); i += blockDim.x) {
     const int up = i % (Z + 1), s = i / (Z + 1) % 2, j = i / (2 * (Z + 1));
     const float e =
@@ -244,7 +247,7 @@ __global__ void __launch_bounds__(256, 4) packed_lattice_kernel(const __grid_con
   else sown = reinterpret_cast<const uint8_t*>(plane + own)[part];
   uint32_t x[Z], cp[4];
 #pragma unroll
-  for (int i = 0; i < Z; ++i) x[i] = __ldg(plane + off[i]);
+  for (int i = 0; i < Z; ++i) x[i] = plane[off[i]];
   bit_counts<Z>(x, cp);
   if constexpr (NP == 3) cp[3] = sown << (LANES * part);
   // nibble m of nib[q] = planes 0..3 of lane 4 m + q
@@ -501,9 +504,9 @@ int launch_word_columns(const sck_plan* plan, const ObsParams& p, cudaStream_t s
 // --------------------------------------------------------------------------------------------- host side
 template <class Lat, bool BARKER>
 static void launch_packed(const WordParams& p, int parts, dim3 grid, cudaStream_t s) {
-  if (parts == 1) packed_lattice_kernel<Lat, 32, BARKER><<<grid, 256, 0, s>>>(p);
-  else if (parts == 2) packed_lattice_kernel<Lat, 16, BARKER><<<grid, 256, 0, s>>>(p);
-  else packed_lattice_kernel<Lat, 8, BARKER><<<grid, 256, 0, s>>>(p);
+  if (parts == 1) launch_dependent(packed_lattice_kernel<Lat, 32, BARKER>, grid, 256, s, p);
+  else if (parts == 2) launch_dependent(packed_lattice_kernel<Lat, 16, BARKER>, grid, 256, s, p);
+  else launch_dependent(packed_lattice_kernel<Lat, 8, BARKER>, grid, 256, s, p);
 }
 
 template <class Lat>
@@ -512,11 +515,11 @@ static void launch_word_t(const sck_plan* plan, const WordParams& p, int parts, 
     if (plan->geom.acceptance == SCK_BARKER) launch_packed<Lat, true>(p, parts, grid, s);
     else launch_packed<Lat, false>(p, parts, grid, s);
   } else if (plan->mode == SCK_MODE_BITWISE) {
-    if (p.c.field) bitwise_shared_lattice_kernel<Lat, true><<<grid, 256, 0, s>>>(p);
-    else bitwise_shared_lattice_kernel<Lat, false><<<grid, 256, 0, s>>>(p);
+    if (p.c.field) launch_dependent(bitwise_shared_lattice_kernel<Lat, true>, grid, 256, s, p);
+    else launch_dependent(bitwise_shared_lattice_kernel<Lat, false>, grid, 256, s, p);
   } else {
-    if (p.c.field) bitwise_independent_lattice_kernel<Lat, true><<<grid, 256, 0, s>>>(p);
-    else bitwise_independent_lattice_kernel<Lat, false><<<grid, 256, 0, s>>>(p);
+    if (p.c.field) launch_dependent(bitwise_independent_lattice_kernel<Lat, true>, grid, 256, s, p);
+    else launch_dependent(bitwise_independent_lattice_kernel<Lat, false>, grid, 256, s, p);
   }
 }
 

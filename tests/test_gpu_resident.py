@@ -60,16 +60,29 @@ def test_resident_lattice_kernels_equal_the_generic_one(name, f32, sweeps):
     assert torch.equal(S, S2)
 
 
-@pytest.mark.parametrize("name", ["ising-square", "ising-sc-open", "ising-fcc", "ising-bcc-j1j2"])
+MARCH = {   # the marching kernel's boxes: words of a row below, at and above a block, chunks with a remainder
+    "march-square": lambda: _sys(1, "square", (36, 54), h=(0.2,)),
+    "march-square-wide": lambda: _sys(1, "square", (1040, 10), acceptance="barker"),
+    "march-sc": lambda: _sys(1, "sc", (8, 4, 18)),
+    "march-sc-large": lambda: _sys(1, "sc", (64, 34, 20), J={1: -1.0}, acceptance="barker"),
+    "march-sc-thin": lambda: _sys(1, "sc", (4, 2, 2), h=(-0.4,)),
+}
+
+
+@pytest.mark.parametrize("name", ["ising-square", "ising-sc-open", "ising-fcc", "ising-bcc-j1j2"] + sorted(MARCH))
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("B", [1, 7, 300])
 def test_ising_class_kernel_equals_the_generic_one(name, f32, B):
-    s = RESIDENT[name]()
+    s = {**RESIDENT, **MARCH}[name]()
     kw = dict(packed=False, spin_dtype=torch.float32 if f32 else torch.int8)
     A, G = (Sampler(s, B, device="cuda", seed=3, **kw) for _ in range(2))
     A.tune(True, 0, 0)
     G.tune(False, 0, 0)
     S = A.init_spins(seed=2)
+    if B == 7:                       # any value counts by its sign; a zero spin stays zero
+        S = torch.randint(-127, 128, S.shape, generator=torch.Generator().manual_seed(1)).to(S)
+        S = S * (A.mask != 0)
+        S = S.to(A.spin_dtype)
     S2 = S.clone()
     for X, Y in ((A, S), (G, S2)):
         X.set_temperature(torch.linspace(1.5, 6.0, B))
