@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
 // before the next chunk overwrites the stage. The epilogue reads the accumulator with tcgen05.ld (warp w reads
 // rows 32 w .. 32 w + 31) and applies bias, ReLU and the bfloat16 conversion.
 constexpr int UM = 128;     // rows per block (MMA M)
-constexpr int UKC = 32;     // K per staged chunk (two K16 MMAs)
+constexpr int UN = 64;                       // output columns of a block
 constexpr long long kUmmaWaitLimit = 1ll << 22;
 
 static __device__ unsigned long long g_made_wait_timeouts;
@@ -262,16 +262,20 @@ __device__ __forceinline__ bool umma_try_wait(uint32_t mbar, uint32_t parity) {
   return ok != 0;
 }
 
-template <int N, int EPI>
+// Grid (M / 128, g.N / N): a block multiplies one 128-row tile by N output columns. Its time is the latency of its
+// loads, so the 256-column layers run as four blocks of 64 columns per row tile: 256 blocks at M = 8192, all resident
+// at once, where 64 blocks of 256 columns left half of the SMs idle behind four times the copies each. K comes in two
+// chunks of KC, one per stage (eight of 32 put a copy's latency between every two products).
+template <int N, int EPI, int KC>
 __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
   // two stages: the copies of chunk ch + 1 run while the tensor cores multiply chunk ch
   extern __shared__ __align__(1024) unsigned char usm[];
-  __nv_bfloat16* As = (__nv_bfloat16*)usm;                                    // [2][UM * UKC]
-  __nv_bfloat16* Bs = (__nv_bfloat16*)(usm + 2 * UM * UKC * 2);               // [2][N * UKC]
-  uint64_t* mbar = (uint64_t*)(usm + 2 * (UM + N) * UKC * 2);                 // [2]
+  __nv_bfloat16* As = (__nv_bfloat16*)usm;                                    // [2][UM * KC]
+  __nv_bfloat16* Bs = (__nv_bfloat16*)(usm + 2 * UM * KC * 2);               // [2][N * KC]
+  uint64_t* mbar = (uint64_t*)(usm + 2 * (UM + N) * KC * 2);                 // [2]
   uint32_t* tmem_slot = (uint32_t*)(mbar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * UM;
+  const int m0 = blockIdx.x * UM, n0 = blockIdx.y * N;
   const uint32_t mb0 = smem_u32(mbar), mb1 = smem_u32(mbar + 1);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
@@ -291,19 +295,19 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
                              ((uint32_t)(UM >> 4) << 24);   // FP32 accumulator, bf16 A and B, K-major
   constexpr uint32_t A_LBO = (UM / 8) * 128, B_LBO = (N / 8) * 128;
-  const int nch = g.K / UKC;
+  const int nch = g.K / KC;
   auto stage = [&](int ch) {
-    const int k0 = ch * UKC, b = ch & 1;
-    __nv_bfloat16* as = As + b * UM * UKC;
-    __nv_bfloat16* bs = Bs + b * N * UKC;
-    for (int i = tid; i < UM * (UKC / 8); i += 128) {
-      const int r = i / (UKC / 8), c = i % (UKC / 8);
+    const int k0 = ch * KC, b = ch & 1;
+    __nv_bfloat16* as = As + b * UM * KC;
+    __nv_bfloat16* bs = Bs + b * N * KC;
+    for (int i = tid; i < UM * (KC / 8); i += 128) {
+      const int r = i / (KC / 8), c = i % (KC / 8);
       cp_async16(as + ((c * (UM / 8) + (r >> 3)) * 64 + (r & 7) * 8), g.A + (long long)(m0 + r) * g.lda + k0 + 8 * c,
                  16);
     }
-    for (int i = tid; i < N * (UKC / 8); i += 128) {
-      const int n = i / (UKC / 8), c = i % (UKC / 8);
-      cp_async16(bs + ((c * (N / 8) + (n >> 3)) * 64 + (n & 7) * 8), g.B + (long long)n * g.ldb + k0 + 8 * c, 16);
+    for (int i = tid; i < N * (KC / 8); i += 128) {
+      const int n = i / (KC / 8), c = i % (KC / 8);
+      cp_async16(bs + ((c * (N / 8) + (n >> 3)) * 64 + (n & 7) * 8), g.B + (long long)(n0 + n) * g.ldb + k0 + 8 * c, 16);
     }
     cp_async_commit();
   };
@@ -340,9 +344,9 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint32_t a_s = smem_u32(As + b * UM * UKC), b_s = smem_u32(Bs + b * N * UKC);
+      const uint32_t a_s = smem_u32(As + b * UM * KC), b_s = smem_u32(Bs + b * N * KC);
 #pragma unroll
-      for (int s = 0; s < UKC / 16; ++s) {
+      for (int s = 0; s < KC / 16; ++s) {
         const uint64_t ad = umma_desc(a_s + s * 2 * A_LBO, A_LBO, 128);
         const uint64_t bd = umma_desc(b_s + s * 2 * B_LBO, B_LBO, 128);
         const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
@@ -373,16 +377,16 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
       float f[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[e]) + g.bias[col + e];
+      for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[e]) + g.bias[n0 + col + e];
       if (EPI == EPI_BIAS_RELU_BF16) {
         uint4 o;
         o.x = pack_bf16(fmaxf(f[0], 0.f), fmaxf(f[1], 0.f));
         o.y = pack_bf16(fmaxf(f[2], 0.f), fmaxf(f[3], 0.f));
         o.z = pack_bf16(fmaxf(f[4], 0.f), fmaxf(f[5], 0.f));
         o.w = pack_bf16(fmaxf(f[6], 0.f), fmaxf(f[7], 0.f));
-        *(uint4*)((__nv_bfloat16*)g.C + (long long)row * g.ldc + col) = o;
+        *(uint4*)((__nv_bfloat16*)g.C + (long long)row * g.ldc + n0 + col) = o;
       } else {
-        float* o = (float*)g.C + (long long)row * g.ldc + col;
+        float* o = (float*)g.C + (long long)row * g.ldc + n0 + col;
         *(float4*)o = make_float4(f[0], f[1], f[2], f[3]);
         *(float4*)(o + 4) = make_float4(f[4], f[5], f[6], f[7]);
       }
@@ -402,8 +406,8 @@ __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
                  : "memory");
 }
 
-template <int N>
-constexpr int umma_smem() { return 2 * (UM + N) * UKC * 2 + 16 + 16; }
+template <int N, int KC>
+constexpr int umma_smem() { return 2 * (UM + N) * KC * 2 + 16 + 16; }
 
 }  // namespace made
 
@@ -417,19 +421,22 @@ int made_set_wait_limit(long long polls) {
 
 namespace made {
 
-template <int N, int EPI>
+template <int N, int EPI, int KC>
 int umma_gemm_n(const GemmArgs& g, cudaStream_t s) {
-  const int rc = cuda_status(cudaFuncSetAttribute(umma_gemm_kernel<N, EPI>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, umma_smem<N>()),
+  const int rc = cuda_status(cudaFuncSetAttribute(umma_gemm_kernel<N, EPI, KC>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, umma_smem<N, KC>()),
                              "made tcgen05 gemm smem");
   if (rc != SCK_OK) return rc;
-  umma_gemm_kernel<N, EPI><<<dim3(g.M / UM), 128, umma_smem<N>(), s>>>(g);
+  umma_gemm_kernel<N, EPI, KC><<<dim3(g.M / UM, g.N / N), 128, umma_smem<N, KC>(), s>>>(g);
   return cuda_status(cudaGetLastError(), "made tcgen05 gemm");
 }
 
 template <int EPI>
 int umma_gemm(const GemmArgs& g, cudaStream_t s) {
-  return g.N == H ? umma_gemm_n<H, EPI>(g, s) : umma_gemm_n<NSP, EPI>(g, s);
+  static_assert(H % UN == 0 && NSP % UN == 0, "whole column tiles");
+  // two chunks, both in flight from the start: half of the 160 inputs, or of the 256 units
+  static_assert(IN % 160 == 0 && H % 256 == 0, "two chunks of whole K16 steps");
+  return g.K == IN ? umma_gemm_n<UN, EPI, 80>(g, s) : umma_gemm_n<UN, EPI, 128>(g, s);
 }
 
 template <bool A_K, bool B_K, int EPI>
@@ -473,13 +480,19 @@ __global__ void loss_kernel(const float* __restrict__ logits, const __nv_bfloat1
   __shared__ float part[8];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = lq;
   __syncthreads();
-  if (threadIdx.x < 4) {
-    const int r = blockIdx.x * 4 + threadIdx.x;
-    const float v = part[2 * threadIdx.x] + part[2 * threadIdx.x + 1];
-    if (r < M) {
-      if (logq) logq[r] = v;
-      if (loss) atomicAdd(loss, -v / (float)M);
+  if (threadIdx.x == 0) {
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = blockIdx.x * 4 + i;
+      const float v = part[2 * i] + part[2 * i + 1];
+      if (r < M) {
+        if (logq) logq[r] = v;
+        sum += v;
+      }
     }
+    // one addition per block: with one per row, 8,192 additions to one address set the kernel's pace
+    if (loss) atomicAdd(loss, -sum / (float)M);
   }
 }
 

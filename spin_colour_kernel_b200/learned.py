@@ -79,13 +79,18 @@ def flatten(params) -> np.ndarray:
     return np.concatenate([np.concatenate([W.reshape(-1), b.reshape(-1)]) for W, b in params]).astype(np.float32)
 
 
-def unflatten(flat: np.ndarray):
+def split(flat: np.ndarray):
+    """[(W, b)] views of one flat parameter array."""
     out, o = [], 0
     for (wshape, bshape) in SHAPES:
         nw, nb = wshape[0] * wshape[1], bshape[0]
-        out.append((flat[o:o + nw].reshape(wshape).copy(), flat[o + nw:o + nw + nb].copy()))
+        out.append((flat[o:o + nw].reshape(wshape), flat[o + nw:o + nw + nb]))
         o += nw + nb
     return out
+
+
+def unflatten(flat: np.ndarray):
+    return [(W.copy(), b.copy()) for W, b in split(flat)]
 
 
 class BlockProposal:
@@ -178,12 +183,13 @@ class BlockProposal:
     def grads(self, x: torch.Tensor):
         """(loss, [(dW, db)] as float32 NumPy) of the mean negative log-density of rows x."""
         n = x.shape[0]
-        g = torch.empty(NPARAM, dtype=torch.float32, device=self.device)
-        loss = torch.empty(1, dtype=torch.float32, device=self.device)
+        # gradients and loss side by side: one copy to the host, whose arrays are handed out as they are
+        out = torch.empty(NPARAM + 1, dtype=torch.float32, device=self.device)
         with torch.cuda.device(self.device):
-            abi.check(abi.lib().sck_made_grads(_ptr(self.params), self.groups, _ptr(x.contiguous()), n, _ptr(g),
-                                               _ptr(loss), _ptr(self._workspace(n)), self._stream()))
-        return float(loss.item()), unflatten(g.cpu().numpy())
+            abi.check(abi.lib().sck_made_grads(_ptr(self.params), self.groups, _ptr(x.contiguous()), n, _ptr(out),
+                                               _ptr(out[NPARAM:]), _ptr(self._workspace(n)), self._stream()))
+        host = out.cpu().numpy()
+        return float(host[NPARAM]), split(host[:NPARAM])
 
     def train(self, data: torch.Tensor, steps: int, batch: int = 8192, lr: float = 1e-3, betas=(0.9, 0.999),
               eps: float = 1e-8, seed: int = 0):
