@@ -484,7 +484,7 @@ int word_column_blocks(const sck_plan* plan, int batch) {
   const int chunk = word_column_chunk(plan, batch);
   const long long items = (long long)((ncol + 255) / 256) * ((len + chunk - 1) / chunk);
   const int words = (batch + 31) / 32;
-  const long long want = (148 * 8 + words - 1) / words;      // more items than that share blocks
+  const long long want = (148 * 16 + words - 1) / words;     // more items than that share blocks
   return (int)(items < want ? items : want);
 }
 
