@@ -102,6 +102,88 @@ __global__ void __launch_bounds__(256) observables_kernel(const __grid_constant_
   }
 }
 
+// The same sums for float32 systems on a lattice table whose bonds carry extra matrices (resident.cu's table match):
+// neighbours at constant offsets, bonds in a compile-time loop. The kernel above spends most of its 1,227 instructions
+// per site of a nanodisk on the run-time bond list and its axis checks (25 us for 64 disks of 39 x 39 x 5).
+template <class Lat, int N>
+__global__ void __launch_bounds__(256) observables_extra_kernel(const __grid_constant__ ObsParams p) {
+  const Geometry& g = p.g;
+  const int rep = blockIdx.y;
+  constexpr int NV = 1 + Lat::b * N;
+  double acc[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) acc[i] = 0.0;
+  for (int site = blockIdx.x * blockDim.x + threadIdx.x; site < g.nsite; site += p.blocks_per_rep * blockDim.x) {
+    if (p.mask != nullptr && p.mask[site] == 0) continue;
+    const int alpha = (int)fdiv((uint32_t)site, p.fd_plane);
+    const int rem = site - alpha * g.plane;
+    const int row = (int)fdiv((uint32_t)rem, p.fd_L1);
+    const int x = rem - row * g.L1;
+    const int z = (int)fdiv((uint32_t)row, p.fd_L2);
+    const int y = row - z * g.L2;
+    double s[N], v[N];
+    load_spin<N, 1>(p, rep, site, s);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = 0.0;
+    const Around<Lat::reach, false> nb(g, x, y, z);
+    static_for<0, Lat::b>([&](auto ac) {
+      constexpr int a = decltype(ac)::value;
+      if (a != alpha) return;
+      static_for<0, Lat::n_bonds(a)>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        constexpr BondC bd = Lat::bond(a, i);
+        if (!nb.valid(bd)) return;
+        double t[N];
+        load_spin<N, 1>(p, rep, nb.index(g, bd), t);
+        const double J = p.obs[a].J[i];
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] += J * t[k];
+        const int e = p.sub[a].bonds[i].extra;
+        if (e >= 0) {
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+#pragma unroll
+            for (int l = 0; l < N; ++l) v[k] += p.obs[a].E[e][3 * k + l] * t[l];
+        }
+      });
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[1 + a * N + k] += s[k];
+    });
+    double e = 0.0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) e += -0.5 * s[k] * v[k] - p.h64[k] * s[k];
+    if constexpr (N == 3) {
+      if (g.has_cubic) {
+        const double k1 = (double)p.k1[site];
+        const double xy = s[0] * s[1], xz = s[0] * s[2], yz = s[1] * s[2], xyz = s[0] * s[1] * s[2];
+        e += k1 * (xy * xy + xz * xz + yz * yz) + p.k2 * xyz * xyz;
+      }
+    }
+    acc[0] += e;
+  }
+  __shared__ double red[NV][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double w = acc[i];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) w += __shfl_down_sync(0xFFFFFFFFu, w, off);
+    if (lane == 0) red[i][warp] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double w = 0.0;
+    for (int wi = 0; wi < (int)(blockDim.x >> 5); ++wi) w += red[threadIdx.x][wi];
+    p.partial[((size_t)rep * p.blocks_per_rep + blockIdx.x) * OBS_VALUES + threadIdx.x] = w;
+  }
+}
+
+template <class Lat>
+static void launch_obs_extra(const ObsParams& p, dim3 grid, cudaStream_t s) {
+  if (p.g.n == 2) observables_extra_kernel<Lat, 2><<<grid, 256, 0, s>>>(p);
+  else observables_extra_kernel<Lat, 3><<<grid, 256, 0, s>>>(p);
+}
+
 // Systems with a compile-time bond table (lattices.h): every neighbour offset is a constant and each bond is
 // visited once, from the end for which it points "forward" (to a higher sublattice, or within a sublattice to a
 // positive offset in z, then y, then x); its reverse sits in the partner's table with the same coupling, so
@@ -744,6 +826,15 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
       case Lat_bcc_1::id: launch_obs_spec<Lat_bcc_1>(p, grid, s); break;
       case Lat_bcc_1_2::id: launch_obs_spec<Lat_bcc_1_2>(p, grid, s); break;
       default: launch_obs_spec<Lat_fcc_1>(p, grid, s); break;
+    }
+  } else if (plan->resident_spec != 0 && p.storage == 1 && n > 1) {   // a table match set aside for its extra matrices
+    switch (plan->resident_spec) {
+      case Lat_square_1::id: launch_obs_extra<Lat_square_1>(p, grid, s); break;
+      case Lat_triangular_1::id: launch_obs_extra<Lat_triangular_1>(p, grid, s); break;
+      case Lat_sc_1::id: launch_obs_extra<Lat_sc_1>(p, grid, s); break;
+      case Lat_bcc_1::id: launch_obs_extra<Lat_bcc_1>(p, grid, s); break;
+      case Lat_bcc_1_2::id: launch_obs_extra<Lat_bcc_1_2>(p, grid, s); break;
+      default: launch_obs_extra<Lat_fcc_1>(p, grid, s); break;
     }
   } else if (obs_columns(plan, storage)) {
     const int rc = launch_word_columns(plan, p, s);
