@@ -1000,14 +1000,16 @@ __global__ void __launch_bounds__(step_threads<G>()) step_kernel(StepParams p) {
 // summation order as in the chain (the extra k-tiles of a chunk meet masked zero weights and add exact zeros), and
 // log q(x) sums its 64 terms in the chain's order, so that the density of a configuration is the same number
 // whether it is drawn or current: the Metropolis-Hastings ratio stays exact to the last bit.
-constexpr int PAIR_TILE_SMEM = WARP_SMEM + 2 * 16 * NSP + 16 * 4;   // + current and proposed spins, log q(x')
+constexpr int PAIR_TILE_SMEM = WARP_SMEM + 2 * 16 * NSP;   // + current and proposed spins
 constexpr int DENSE_CHUNKS = 26;      // 8 per hidden layer (32 units each), 2 for the output layer
 // the dense pass splits the two slice buffers into three chunk buffers, so that two chunks load while one is used
 constexpr int DENSE_BUF_ELEMS = 2 * 13248 / 3;
 static_assert(3 * DENSE_BUF_ELEMS == 2 * Slice<16>::ELEMS, "three chunk buffers fill the two slice buffers");
 static_assert(32 * HS <= DENSE_BUF_ELEMS && 32 * XS <= DENSE_BUF_ELEMS, "a chunk fits its buffer");
 
-constexpr int pair_smem() { return STEP_WARPS * PAIR_TILE_SMEM + 2 * Slice<16>::BYTES; }
+constexpr int pair_smem() {
+  return STEP_WARPS * PAIR_TILE_SMEM + 2 * Slice<16>::BYTES + ((int)sizeof(Tables) + 15) / 16 * 16;
+}
 
 struct DenseChunk {
   int layer, u0, nkt, ld;
@@ -1046,7 +1048,7 @@ __device__ __forceinline__ void load_dense_chunk(__nv_bfloat16* dst, const StepP
 }
 
 // Grid of persistent blocks of 5 tiles x 2 warps; tile rows r = 0..15 are the proposals of blocks 16 t + r, lanes
-// (gr, q) of the tile's first warp own blocks gr and gr + 8 for the draws, densities, energy and write-back.
+// (gr, q) of the tile's warp w own block gr + 8 w for the draws, densities, energy and write-back.
 __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepParams p) {
   using SL = Slice<16>;
   constexpr int U = SL::U, S = SL::S;
@@ -1059,17 +1061,19 @@ __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepPara
   int8_t* const CUR = (int8_t*)(tbase + WARP_SMEM);           // [16][64] current spins of the tile's blocks
   int8_t* const PROP = CUR + 16 * NSP;                        // [16][64] proposed spins
   float* const LS = (float*)H0;   // [16][64] log-sigmoid terms of x, over layer 1's activations once they are spent
-  float* const LQN = (float*)(PROP + 16 * NSP);               // [16] log q(x') of the rows the second warp drew
   __nv_bfloat16* const slices = (__nv_bfloat16*)(smem + STEP_WARPS * PAIR_TILE_SMEM);
   for (int i = lane + 32 * sub; i < WARP_SMEM / 16; i += 64) ((uint4*)X)[i] = make_uint4(0, 0, 0, 0);
-  tile_sync(warp, 2);
+  // the geometry tables beside the slices: their indices differ between lane groups, which constant loads serialise
+  Tables& tab = *(Tables*)(smem + STEP_WARPS * PAIR_TILE_SMEM + 2 * SL::BYTES);
+  for (int i = threadIdx.x; i < (int)sizeof(Tables); i += blockDim.x) ((int8_t*)&tab)[i] = ((const int8_t*)&c_tab)[i];
+  __syncthreads();
 
   const long long tasks = (long long)p.R * p.nc;
   const long long ctasks = (tasks + 16 * STEP_WARPS - 1) / (16 * STEP_WARPS);   // 16 blocks per tile
   const int half = p.nb >> 1, L = p.L;
   if ((long long)blockIdx.x < ctasks) load_slice<16>(slices, p, 0);
   for (long long ct = blockIdx.x; ct < ctasks; ct += gridDim.x) {
-    tile_sync(warp, 2);   // the first warp is done with the previous blocks' rows
+    tile_sync(warp, 2);   // both warps are done with the previous blocks' rows
     const bool more = ct + gridDim.x < ctasks;
     // ---- gather: row r = block 16 (ct * tiles + tile) + r; both warps, rows split by lane group and warp
     for (int rr = 0; rr < 2; ++rr) {
@@ -1081,38 +1085,40 @@ __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepPara
       const int bx = 2 * (k % half) + (p.colour & 1), by = 2 * (k / half % half) + ((p.colour >> 1) & 1),
                 bz = 2 * (k / (half * half)) + (p.colour >> 2);
       const int8_t* base = p.spins + (long long)rep * L * L * L;
-      for (int col = q + 4 * sub; col < IN; col += 8) {
-        float s = 0.f;
-        if (valid) {
-          const int x = wrap_block(4 * bx + c_tab.in_off[col][0], L), y = wrap_block(4 * by + c_tab.in_off[col][1], L),
-                    z = wrap_block(4 * bz + c_tab.in_off[col][2], L);
-          s = (float)base[((long long)z * L + y) * L + x];
+      // ten loads in flight a time
+#pragma unroll 1
+      for (int c0 = q + 4 * sub; c0 < IN; c0 += 80) {
+        int8_t v[10];
+#pragma unroll
+        for (int i = 0; i < 10; ++i) {
+          const int col = c0 + 8 * i;
+          v[i] = 0;
+          if (valid) {
+            const int x = wrap_block(4 * bx + tab.in_off[col][0], L), y = wrap_block(4 * by + tab.in_off[col][1], L),
+                      z = wrap_block(4 * bz + tab.in_off[col][2], L);
+            v[i] = base[((long long)z * L + y) * L + x];
+          }
         }
-        X[r * XS + col] = col < NBD ? __float2bfloat16_rn(s) : __float2bfloat16_rn(0.f);
-        if (col >= NBD) CUR[r * NSP + col - NBD] = (int8_t)(int)s;
+#pragma unroll
+        for (int i = 0; i < 10; ++i) {
+          const int col = c0 + 8 * i;
+          X[r * XS + col] = col < NBD ? __float2bfloat16_rn((float)v[i]) : __float2bfloat16_rn(0.f);
+          if (col >= NBD) CUR[r * NSP + col - NBD] = v[i];
+        }
       }
     }
     __syncwarp();
     tile_sync(warp, 2);
 
-    // ---- the first warp's two blocks
-    long long task2[2];
-    bool valid2[2];
-    int rep2[2], b3[2][3];
-    long long uid2[2];
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      task2[rr] = (ct * STEP_WARPS + warp) * 16 + gr + 8 * rr;
-      valid2[rr] = task2[rr] < tasks;
-      rep2[rr] = valid2[rr] ? (int)(task2[rr] / p.nc) : 0;
-      const int k = valid2[rr] ? (int)(task2[rr] % p.nc) : 0;
-      b3[rr][0] = 2 * (k % half) + (p.colour & 1);
-      b3[rr][1] = 2 * (k / half % half) + ((p.colour >> 1) & 1);
-      b3[rr][2] = 2 * (k / (half * half)) + (p.colour >> 2);
-      uid2[rr] = (long long)rep2[rr] * p.nb * p.nb * p.nb + (b3[rr][0] + p.nb * (b3[rr][1] + p.nb * b3[rr][2]));
-    }
-    // warp `sub` draws the spins of rows gr + 8 sub (block uid_mine)
-    const long long uid_mine = sub ? uid2[1] : uid2[0];
+    // ---- warp `sub` draws, judges and writes back the blocks of rows gr + 8 sub, one per lane group
+    const int r = gr + 8 * sub;
+    const long long task = (ct * STEP_WARPS + warp) * 16 + r;
+    const bool valid = task < tasks;
+    const int rep = valid ? (int)(task / p.nc) : 0;
+    const int k = valid ? (int)(task % p.nc) : 0;
+    const int bx = 2 * (k % half) + (p.colour & 1), by = 2 * (k / half % half) + ((p.colour >> 1) & 1),
+              bz = 2 * (k / (half * half)) + (p.colour >> 2);
+    const long long uid_mine = (long long)rep * p.nb * p.nb * p.nb + (bx + p.nb * (by + p.nb * bz));
     float lq_mine = 0.f;
     // ---- the autoregressive chain: 16 steps of 4 spins
     for (int g = 0; g < 16; ++g) {
@@ -1169,8 +1175,7 @@ __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepPara
     }
     lq_mine += __shfl_xor_sync(0xffffffffu, lq_mine, 1);
     lq_mine += __shfl_xor_sync(0xffffffffu, lq_mine, 2);
-    if (sub == 1 && q == 0) LQN[gr + 8] = lq_mine;
-    tile_sync(warp, 2);   // the last draws are in X, the second warp's densities in LQN
+    tile_sync(warp, 2);   // the last draws are in X
     // ---- keep the proposals, put the current spins in their place
     for (int i = lane + 32 * sub; i < 16 * NSP; i += 64) {
       const int r = i / NSP, j = i - r * NSP;
@@ -1217,74 +1222,67 @@ __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepPara
     }
     __syncthreads();   // every warp is done with the chunk buffers and the terms of log q(x) are in place
     if (more) load_slice<16>(slices, p, 0);
-    if (sub != 0) continue;   // densities, energy change, acceptance and write-back: the tile's first warp
+    // ---- densities, energy change, acceptance and write-back, each warp its own rows
     // log q(x) in the chain's order: lane q < 2 adds positions 4 g + 2 q, 4 g + 2 q + 1 for g = 0 .. 15
-    float lq_old[2] = {0.f, 0.f};
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      if (q < 2)
-        for (int g = 0; g < 16; ++g) {
-          lq_old[rr] += LS[(gr + 8 * rr) * NSP + 4 * g + 2 * q];
-          lq_old[rr] += LS[(gr + 8 * rr) * NSP + 4 * g + 2 * q + 1];
-        }
-      lq_old[rr] += __shfl_xor_sync(0xffffffffu, lq_old[rr], 1);
-      lq_old[rr] += __shfl_xor_sync(0xffffffffu, lq_old[rr], 2);
+    float lqo = 0.f;
+    if (q < 2)
+      for (int g = 0; g < 16; ++g) {
+        lqo += LS[r * NSP + 4 * g + 2 * q];
+        lqo += LS[r * NSP + 4 * g + 2 * q + 1];
+      }
+    lqo += __shfl_xor_sync(0xffffffffu, lqo, 1);
+    lqo += __shfl_xor_sync(0xffffffffu, lqo, 2);
+    const float lqn = lq_mine;
+    // energy change, integer: -(sum_internal (x'x' - xx) + sum_face (x' - x) b)
+    const int8_t* xn_row = PROP + r * NSP;
+    const int8_t* xc_row = CUR + r * NSP;
+    int de = 0;
+#pragma unroll 4
+    for (int i = q; i < 144; i += 4) {
+      const int a = tab.internal[i][0], b = tab.internal[i][1];
+      de -= (int)xn_row[a] * (int)xn_row[b] - (int)xc_row[a] * (int)xc_row[b];
     }
+#pragma unroll 4
+    for (int i = q; i < NBD; i += 4) {
+      const int a = tab.face[i];
+      const int bd = (int)__bfloat162float(X[r * XS + i]);
+      de -= ((int)xn_row[a] - (int)xc_row[a]) * bd;
+    }
+    de += __shfl_xor_sync(0xffffffffu, de, 1);
+    de += __shfl_xor_sync(0xffffffffu, de, 2);
+    int acc_flag = 0;
+    if (q == 0 && valid) {
+      const Philox4 ra = philox4x32_10((uint32_t)(int32_t)(17 * uid_mine + 16), 0u, p.k0, p.k1);
+      const float ua = to_uniform(ra.x0);
+      const float logr = -p.beta[rep] * (float)de + lqo - lqn;
+      acc_flag = ua < __expf(fminf(logr, 0.f)) ? 1 : 0;
+      if (acc_flag && p.accepted) atomicAdd(p.accepted + rep, 1);
+    }
+    acc_flag = __shfl_sync(0xffffffffu, acc_flag, lane & ~3);
+    if (valid && acc_flag) {
+      // lane q writes the four x-rows of layer lz = q
+      int8_t* dst = p.spins + (long long)rep * L * L * L;
+      const int x0 = 4 * bx, y0 = 4 * by, z0 = 4 * bz;
 #pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      const int r = gr + 8 * rr;
-      const float lqn = rr ? LQN[r] : lq_mine;
-      const float lqo = lq_old[rr];
-      // energy change, integer: -(sum_internal (x'x' - xx) + sum_face (x' - x) b)
-      const int8_t* xn_row = PROP + r * NSP;
-      const int8_t* xc_row = CUR + r * NSP;
-      int de = 0;
-      for (int i = q; i < 144; i += 4) {
-        const int a = c_tab.internal[i][0], b = c_tab.internal[i][1];
-        de -= (int)xn_row[a] * (int)xn_row[b] - (int)xc_row[a] * (int)xc_row[b];
-      }
-      for (int i = q; i < NBD; i += 4) {
-        const int a = c_tab.face[i];
-        const int bd = (int)__bfloat162float(X[r * XS + i]);
-        de -= ((int)xn_row[a] - (int)xc_row[a]) * bd;
-      }
-      de += __shfl_xor_sync(0xffffffffu, de, 1);
-      de += __shfl_xor_sync(0xffffffffu, de, 2);
-      const bool valid = valid2[rr];
-      const int rep = rep2[rr];
-      int acc_flag = 0;
-      if (q == 0 && valid) {
-        const Philox4 ra = philox4x32_10((uint32_t)(int32_t)(17 * uid2[rr] + 16), 0u, p.k0, p.k1);
-        const float ua = to_uniform(ra.x0);
-        const float logr = -p.beta[rep] * (float)de + lqo - lqn;
-        acc_flag = ua < __expf(fminf(logr, 0.f)) ? 1 : 0;
-        if (acc_flag && p.accepted) atomicAdd(p.accepted + rep, 1);
-      }
-      acc_flag = __shfl_sync(0xffffffffu, acc_flag, lane & ~3);
-      if (valid && acc_flag) {
-        // lane q writes the four x-rows of layer lz = q
-        int8_t* dst = p.spins + (long long)rep * L * L * L;
-        const int x0 = 4 * b3[rr][0], y0 = 4 * b3[rr][1], z0 = 4 * b3[rr][2];
-        for (int ly = 0; ly < 4; ++ly) {
-          uint32_t word = 0;
+      for (int ly = 0; ly < 4; ++ly) {
+        uint32_t word = 0;
 #pragma unroll
-          for (int lx = 0; lx < 4; ++lx) {
-            const int pos = c_tab.pos_of_raster[lx + 4 * ly + 16 * q];
-            word |= (uint32_t)(uint8_t)xn_row[pos] << (8 * lx);
-          }
-          *(uint32_t*)(dst + ((long long)(z0 + q) * L + (y0 + ly)) * L + x0) = word;
+        for (int lx = 0; lx < 4; ++lx) {
+          const int pos = tab.pos_of_raster[lx + 4 * ly + 16 * q];
+          word |= (uint32_t)(uint8_t)xn_row[pos] << (8 * lx);
         }
+        *(uint32_t*)(dst + ((long long)(z0 + q) * L + (y0 + ly)) * L + x0) = word;
       }
-      if (valid && p.record) {
-        unsigned char* rec = p.record + 80 * task2[rr];
-        for (int pos = q; pos < NSP; pos += 4) rec[pos] = (unsigned char)xn_row[pos];
-        if (q == 0) {
-          float* f = (float*)(rec + NSP);
-          f[0] = lqn;
-          f[1] = lqo;
-          f[2] = (float)de;
-          f[3] = (float)acc_flag;
-        }
+    }
+    if (valid && p.record) {
+      unsigned char* rec = p.record + 80 * task;
+      for (int pos = q; pos < NSP; pos += 4) rec[pos] = (unsigned char)xn_row[pos];
+      if (q == 0) {
+        float* f = (float*)(rec + NSP);
+        f[0] = lqn;
+        f[1] = lqo;
+        f[2] = (float)de;
+        f[3] = (float)acc_flag;
       }
     }
     __syncwarp();
