@@ -622,7 +622,8 @@ def main():
                              f"step times from CUDA events"},
         "e2e": {"value": e2e, "unit": "attempts/ns", "h2d_bytes_per_step": int(beta_h.numel() * 4),
                 "d2h_bytes_per_step": int((E_h.numel() + M_h.numel()) * 8)},
-        "gpu_launches": int(launches + (1 if path["resident"] or groups else K)),
+        # the counter advances once per call; the tile and generic kernels advance it every sweep
+        "gpu_launches": int(launches + (K if args.path in ("tile", "generic") and not path["resident"] else 1)),
         "clocks": clk,
     }
     if rank == 0 and not args.no_cpu_baseline:
