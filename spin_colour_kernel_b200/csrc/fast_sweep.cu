@@ -22,9 +22,11 @@ namespace sck {
 // ------------------------------------------------------------------------------------------------- kernels
 // Grid (ceil(rows * bx / 256), n_tasks * units_per_task). Block y-slot -> (task, `pairs` replica pairs): a thread forms
 // its class site, its neighbours' offsets and the sweep's key once for all of them. Bound by instruction issue (304
-// instructions per attempt with one pair a thread, 75 % of the issue slots, on Heisenberg bcc 32^3 x 2).
+// instructions per attempt with one pair a thread, 75 % of the issue slots, on Heisenberg bcc 32^3 x 2). Five blocks
+// per SM: attempts/ns without a bound / at four / five / six, Heisenberg bcc J1-J2 64^3 x 2 x 64: 60 / 67 / 69 / 60;
+// XY square 512^2 x 33: 157 / 157 / 162 / 160; the quick-start case 511 / 474 / 482 / 475 us.
 template <class Lat, int N, typename ST, bool PER, int NSL>
-__global__ void __launch_bounds__(256) spec_task_kernel(const __grid_constant__ SpecParams p) {
+__global__ void __launch_bounds__(256, 5) spec_task_kernel(const __grid_constant__ SpecParams p) {
   follow_previous();
   const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
