@@ -462,7 +462,7 @@ __global__ void prepare_kernel(const float* __restrict__ master, __nv_bfloat16* 
 
 // loss, log q and the logit gradient -x sigmoid(-x l) / M (bfloat16) of rows of logits
 __global__ void loss_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ x, int M,
-                            __nv_bfloat16* __restrict__ grad, float* __restrict__ logq, float* __restrict__ loss) {
+                            __nv_bfloat16* __restrict__ grad, float* __restrict__ logq, double* __restrict__ lpart) {
   const int row = blockIdx.x * 4 + (threadIdx.x >> 6);
   const int p = threadIdx.x & 63;
   float lq = 0.f;
@@ -481,18 +481,19 @@ __global__ void loss_kernel(const float* __restrict__ logits, const __nv_bfloat1
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = lq;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float sum = 0.f;
+    double sum = 0.0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = blockIdx.x * 4 + i;
       const float v = part[2 * i] + part[2 * i + 1];
       if (r < M) {
         if (logq) logq[r] = v;
-        sum += v;
+        sum += (double)v;
       }
     }
-    // one addition per block: with one per row, 8,192 additions to one address set the kernel's pace
-    if (loss) atomicAdd(loss, -sum / (float)M);
+    // the block's rows to a partial of its own, which finish_kernel adds up in a fixed order in FP64 (8,192 atomic
+    // additions to one FP32 address set this kernel's pace before, and left the loss 1e-6 from run to run)
+    if (lpart) lpart[blockIdx.x] = sum;
   }
 }
 
@@ -549,10 +550,25 @@ struct FinishArgs {
   float* m1;
   float* m2;
   __nv_bfloat16* bf;
+  const double* lpart;     // sums of log q over four rows each, n_lpart of them; loss = -sum / rows (may be null)
+  int n_lpart, rows;
+  float* loss;
   float lr, beta1, beta2, eps, c1, c2;   // c1 = 1 - beta1^t, c2 = 1 - beta2^t
 };
 
-__global__ void finish_kernel(FinishArgs a) {
+__global__ void __launch_bounds__(256) finish_kernel(FinishArgs a) {
+  if (blockIdx.x == 0 && a.loss != nullptr) {
+    __shared__ double red[256];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < a.n_lpart; i += 256) s += a.lpart[i];
+    red[threadIdx.x] = s;
+#pragma unroll
+    for (int h = 128; h > 0; h >>= 1) {
+      __syncthreads();
+      if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+    }
+    if (threadIdx.x == 0) *a.loss = (float)(-red[0] / (double)a.rows);
+  }
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NPARAM) return;
   int l = 3;
@@ -1310,7 +1326,7 @@ __global__ void __launch_bounds__(32 * STEP_WARPS * 2) step_pair_kernel(StepPara
 
 // ======================================================================================= workspace layout
 struct TrainLayout {
-  long long h[3], logits, g4, gh[3], wpart[4], bpart[4], grads, total;
+  long long h[3], logits, g4, gh[3], wpart[4], bpart[4], lpart, total;
   int splits, chunk;   // the weight gradients reduce the batch in `splits` chunks of `chunk` rows (multiple of 64)
 };
 
@@ -1334,7 +1350,7 @@ inline TrainLayout train_layout(int M) {
   for (int l = 0; l < 3; ++l) t.gh[l] = take((long long)M * H * 2);
   for (int l = 0; l < 4; ++l) t.wpart[l] = take((long long)t.splits * out_rows(l) * in_cols(l) * 4);
   for (int l = 0; l < 4; ++l) t.bpart[l] = take((long long)t.splits * out_rows(l) * 4);
-  t.grads = take(NPARAM * 4);
+  t.lpart = take((long long)(M + 3) / 4 * 8);
   t.total = o;
   return t;
 }
@@ -1512,23 +1528,24 @@ int sck_made_forward(const void* params, int32_t groups, const uint16_t* x, int3
   return rc;
 }
 
-static int grads_common(const void* params, int groups, const uint16_t* x, int batch, float* loss, char* ws,
-                        const TrainLayout& t, cudaStream_t s) {
+static int grads_common(const void* params, int groups, const uint16_t* x, int batch, char* ws, const TrainLayout& t,
+                        cudaStream_t s) {
   int rc = forward_layers(params, (const __nv_bfloat16*)x, batch, ws, t, s);
   if (rc) return rc;
-  if (loss) {
-    rc = cuda_status(cudaMemsetAsync(loss, 0, 4, s), "made loss");
-    if (rc) return rc;
-  }
   loss_kernel<<<(batch + 3) / 4, 256, 0, s>>>((const float*)(ws + t.logits), (const __nv_bfloat16*)x, batch,
-                                               (__nv_bfloat16*)(ws + t.g4), nullptr, loss);
+                                               (__nv_bfloat16*)(ws + t.g4), nullptr,
+                                               (double*)(ws + t.lpart));
   rc = cuda_status(cudaGetLastError(), "made loss");
   if (rc) return rc;
   return backward(params, (const __nv_bfloat16*)x, batch, ws, t, s);
 }
 
-static FinishArgs finish_args(char* ws, const TrainLayout& t, int groups) {
+static FinishArgs finish_args(char* ws, const TrainLayout& t, int groups, int batch, float* loss) {
   FinishArgs a{};
+  a.lpart = (const double*)(ws + t.lpart);
+  a.n_lpart = (batch + 3) / 4;
+  a.rows = batch;
+  a.loss = loss;
   for (int l = 0; l < 4; ++l) {
     a.wpart[l] = (const float*)(ws + t.wpart[l]);
     a.bpart[l] = (const float*)(ws + t.bpart[l]);
@@ -1547,9 +1564,9 @@ int sck_made_grads(const void* params, int32_t groups, const uint16_t* x, int32_
   cudaStream_t s = (cudaStream_t)stream;
   const TrainLayout t = train_layout(batch);
   char* ws = (char*)workspace;
-  int rc = grads_common(params, groups, x, batch, loss, ws, t, s);
+  int rc = grads_common(params, groups, x, batch, ws, t, s);
   if (rc) return rc;
-  FinishArgs a = finish_args(ws, t, groups);
+  FinishArgs a = finish_args(ws, t, groups, batch, loss);
   a.adam = 0;
   a.grads = grads;
   finish_kernel<<<(unsigned)((NPARAM + 255) / 256), 256, 0, s>>>(a);
@@ -1567,9 +1584,9 @@ int sck_made_train_step(void* params, float* adam, int32_t groups, const uint16_
   cudaStream_t s = (cudaStream_t)stream;
   const TrainLayout t = train_layout(batch);
   char* ws = (char*)workspace;
-  int rc = grads_common(params, groups, x, batch, loss, ws, t, s);
+  int rc = grads_common(params, groups, x, batch, ws, t, s);
   if (rc) return rc;
-  FinishArgs a = finish_args(ws, t, groups);
+  FinishArgs a = finish_args(ws, t, groups, batch, loss);
   a.adam = 1;
   a.master = (float*)params;
   a.m1 = adam;
