@@ -43,6 +43,8 @@ RESIDENT_LIMIT = 200 << 10        # the plan's default: replicas up to 200 KiB s
 BYTES_PER_ATTEMPT = {"heisenberg-bcc": 24, "ising-sc-bitwise": 0.25, "ising-square": 2, "xy-ragged": 16,
                      "learned-ising-sc": 2}
 FALLBACK_HBM_GBS = 6650.0
+KERNEL_KINDS = ["generic", "lattice", "segment", "tile", "interleaved", "word", "resident lattice", "resident list",
+                "marching"]       # sck_plan_path's kernel kinds (include/sck.h)
 
 
 # ------------------------------------------------------------------------------------------------ workloads
@@ -617,7 +619,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
                      "note": f"algorithmic {bpa} B/attempt; peak {peak_kind}; kernel = "
-                             f"{'bitwise' if A.bitwise else ['generic', 'lattice', 'segment', 'tile', 'interleaved'][path['specialised'] // 100]} class update, "
+                             f"{'bitwise' if A.bitwise else KERNEL_KINDS[path['specialised'] // 100]} class update, "
                              f"{launches_per_sweep} launches per sweep (L2 group {path['group']}), "
                              f"step times from CUDA events"},
         "e2e": {"value": e2e, "unit": "attempts/ns", "h2d_bytes_per_step": int(beta_h.numel() * 4),

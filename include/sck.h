@@ -153,8 +153,10 @@ int sck_plan_shape(const sck_plan* plan, int32_t* computed_replicas, int32_t* ro
  *                         sck_plan_destroy. Call it outside stream capture;
  *   resident_limit_bytes  replicas up to this size (int8 / float32 storage) run all sweeps of a call in shared
  *                         memory, one block per replica; 0 disables it (default 200 KiB, at most 220 KiB).
- * sck_plan_path reports the chosen path: specialised = 100 * kernel kind (1 lattice, 2 segment, 3 tile) + table
- * id (0 = generic), budget, pipeline group (replicas per group; 0 = class by class over all replicas) and whether
+ * sck_plan_path reports the chosen path: specialised = 100 * kernel kind + table id (0 = generic), the kinds being
+ * 1 lattice, 2 segment, 3 tile, 4 interleaved, 5 word storage, 6 resident with constant neighbour offsets (calls of
+ * several sweeps too), 7 resident, calls of four and more sweeps from neighbour lists, 8 marching words (int8 Ising on
+ * two-colour boxes; spins that do not start on 4 bytes take kind 1); budget, pipeline group (replicas per group; 0 = class by class over all replicas) and whether
  * sweeps run resident. No counterpart in the
  * reference, whose Triton launch geometry plays this role (Sampler.__init__,
  * sampler.py:84-115). */

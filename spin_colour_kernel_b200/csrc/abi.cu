@@ -350,6 +350,7 @@ int sck_plan_create(const sck_system_desc* d, int32_t batch, int32_t mode, sck_p
   p->spec = find_spec(p);
   p->word_spec = find_word_spec(p);
   p->resident_spec = find_resident_spec(p);
+  p->resident_lists = resident_lists_ok(p) ? 1 : 0;
   if (mode == SCK_MODE_QUAD) {
     std::string why;
     if (!quad_ok(p, &why)) {
@@ -394,6 +395,7 @@ int sck_plan_tune(sck_plan* plan, int32_t specialised, int64_t l2_budget_bytes, 
   plan->spec = (specialised || plan->mode == SCK_MODE_QUAD) ? find_spec(plan) : 0;   // interleaved: always
   plan->word_spec = specialised ? find_word_spec(plan) : 0;
   plan->resident_spec = specialised ? find_resident_spec(plan) : 0;
+  plan->resident_lists = resident_lists_ok(plan) ? 1 : 0;
   plan->kernel_kind = specialised >= 3 ? 3 : (specialised >= 2 ? 2 : 1);
   plan->l2_budget = l2_budget_bytes;
   plan->resident_limit = resident_limit_bytes;
@@ -429,8 +431,19 @@ int sck_plan_path(const sck_plan* plan, int32_t* specialised, int64_t* l2_budget
   if (plan == nullptr) return fail(SCK_ERR_INVALID, "null plan");
   if (specialised) {
     int kind = pipeline_group(plan) > 0 ? 1 : (tile_kernel_ok(plan) ? 3 : (seg_kernel_ok(plan) ? 2 : 1));
-    if (plan->mode == SCK_MODE_QUAD) kind = 4;
-    *specialised = plan->spec ? kind * 100 + plan->spec : 0;
+    int table = plan->spec;
+    if (plan->mode == SCK_MODE_QUAD) {
+      kind = 4;
+    } else if (use_resident(plan)) {
+      kind = plan->resident_lists ? 7 : 6;
+      table = plan->resident_spec;
+    } else if (plan->word_spec) {
+      kind = 5;
+      table = plan->word_spec;
+    } else if (pipeline_group(plan) == 0 && ising_march_plan(plan)) {
+      kind = 8;
+    }
+    *specialised = table ? kind * 100 + table : 0;
   }
   if (l2_budget_bytes) *l2_budget_bytes = plan->l2_budget;
   if (group) *group = plan->mode == SCK_MODE_QUAD ? 4 * plan->quad_group : pipeline_group(plan);

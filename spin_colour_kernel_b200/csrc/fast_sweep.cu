@@ -480,11 +480,9 @@ static void launch_ising_t(const sck_plan* plan, const IsingClassParams& p, dim3
   }
 }
 
-// The marching kernel's systems: the walk and both row directions alternate between the two colours; its 4-byte loads
-// need spins that start on 4 bytes.
-static bool ising_march_ok(const sck_plan* plan, const void* spins, int colour) {
+// The marching kernel's systems: the walk and both row directions alternate between the two colours.
+bool ising_march_plan(const sck_plan* plan) {
   const Geometry& g = plan->geom;
-  if (colour > 1 || ((uintptr_t)spins & 3u) != 0) return false;
   if (plan->mode != SCK_MODE_INT8 || g.has_mask || g.L1 % 4 != 0 || !spec_periodic_box(plan)) return false;
   if (plan->spec != Lat_square_1::id && plan->spec != Lat_sc_1::id) return false;
   const Colouring& col = plan->col;
@@ -492,6 +490,11 @@ static bool ising_march_ok(const sck_plan* plan, const void* spins, int colour) 
   for (int k = 0; k < g.dim; ++k)
     if (col.K[0][k] != 1) return false;
   return true;
+}
+
+// Its 4-byte loads need spins that start on 4 bytes.
+static bool ising_march_ok(const sck_plan* plan, const void* spins, int colour) {
+  return colour <= 1 && ((uintptr_t)spins & 3u) == 0 && ising_march_plan(plan);
 }
 
 // Chunks of the walk: long ones convert fewer words twice, short ones keep 16 blocks per SM; at least 8 sites.

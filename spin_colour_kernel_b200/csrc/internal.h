@@ -133,6 +133,7 @@ struct sck_plan {
   int spec;        // id of the matching compile-time lattice table (lattices.h), 0 = generic kernels
   int word_spec;   // the same for word storage (words.cu), 0 = the kernels of sweep.cu and bitwise.cu
   int resident_spec;  // the same for resident sweeps (resident.cu), 0 = the resident kernel of sweep.cu
+  int resident_lists; // resident calls of several sweeps run from neighbour lists
   int kernel_kind; // specialised class kernels: 1 lattice, 2 segment (segment.cu), 3 tile (tile.cu) where eligible
   long long l2_budget;  // bytes of L2 the group pipeline may fill
   long long resident_limit;  // largest replica (bytes) whose sweeps run resident in shared memory; 0 = never
@@ -191,6 +192,8 @@ int launch_unpack(const sck_plan* plan, const int32_t* words, const int8_t* mask
 int launch_advance(int64_t* state, int n, cudaStream_t s);
 int match_lattice(const sck_plan* plan, bool extras = false);
 int find_resident_spec(const sck_plan* plan);
+bool resident_lists_ok(const sck_plan* plan);
+bool ising_march_plan(const sck_plan* plan);
 int launch_lattice_resident(const sck_plan* plan, const Common& c, int n_sweeps, cudaStream_t s);
 int lattice_periodic_box(const sck_plan* plan, int id);
 int find_spec(const sck_plan* plan);

@@ -9,6 +9,8 @@
 // in registers, the sweeps' keys are formed 32 at a time and the Ising table row sits beside the spins.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "site.cuh"
 #include "words.cuh"
 
@@ -424,9 +426,34 @@ int find_resident_spec(const sck_plan* plan) {
 constexpr int kListSweeps = 4;
 constexpr size_t kResidentSmem = 222 << 10;
 
-template <class Lat>
-static size_t list_bytes(const LatticeResidentParams& p, int nsite) {
-  return (size_t)p.spin_bytes + (size_t)16 * list_words<Lat>() * nsite + sizeof(float) * p.table_floats;
+// Entries of a replica's Ising table row kept in shared memory beside the spins, 0 none.
+static int table_floats(const sck_plan* plan) {
+  if (plan->geom.n != 1) return 0;
+  const size_t spins = (resident_bytes(plan) + 15) / 16 * 16;
+  const int floats = plan->geom.b * plan->keys;
+  return floats <= 2048 && spins + 4 * (size_t)floats <= (220 << 10) ? floats : 0;
+}
+
+// Spins in slot order with the slot of missing neighbours; the same bytes hold two per site during set-up.
+static size_t list_spin_bytes(const sck_plan* plan) {
+  const int nsite = plan->geom.nsite;
+  const size_t spins = (size_t)plan->geom.n * (nsite + 1) * (plan->mode == SCK_MODE_INT8 ? 1 : 4);
+  return (std::max(spins, (size_t)2 * nsite) + 15) / 16 * 16;
+}
+
+static size_t list_bytes(const sck_plan* plan) {
+  const int words = plan->resident_spec == Lat_square_1::id       ? list_words<Lat_square_1>()
+                    : plan->resident_spec == Lat_triangular_1::id ? list_words<Lat_triangular_1>()
+                    : plan->resident_spec == Lat_sc_1::id         ? list_words<Lat_sc_1>()
+                    : plan->resident_spec == Lat_bcc_1::id        ? list_words<Lat_bcc_1>()
+                    : plan->resident_spec == Lat_bcc_1_2::id      ? list_words<Lat_bcc_1_2>()
+                                                                  : list_words<Lat_fcc_1>();
+  return list_spin_bytes(plan) + (size_t)16 * words * plan->geom.nsite + sizeof(float) * table_floats(plan);
+}
+
+// Calls of kListSweeps sweeps and more run from neighbour lists: 16-bit slots, everything in shared memory.
+bool resident_lists_ok(const sck_plan* plan) {
+  return plan->resident_spec != 0 && plan->geom.nsite < 65535 && list_bytes(plan) <= kResidentSmem;
 }
 
 template <class K>
@@ -457,11 +484,10 @@ static int block_threads(int sites) {
 template <class Lat, int N, typename ST, bool PER>
 static int launch_lattice_resident_t(const sck_plan* plan, LatticeResidentParams& p, cudaStream_t s) {
   const int per = p.c.rows * p.c.bx, B = p.c.B;
-  LatticeResidentParams q = p;
-  q.spin_bytes = (int)(((size_t)N * (plan->geom.nsite + 1) * sizeof(ST) + 15) / 16 * 16);
-  if (q.spin_bytes < 2 * plan->geom.nsite) q.spin_bytes = (2 * plan->geom.nsite + 15) / 16 * 16;
-  const size_t smem = list_bytes<Lat>(q, plan->geom.nsite);
-  if (p.n_sweeps >= kListSweeps && plan->geom.nsite < 65535 && smem <= kResidentSmem) {
+  if (p.n_sweeps >= kListSweeps && plan->resident_lists) {
+    LatticeResidentParams q = p;
+    q.spin_bytes = (int)list_spin_bytes(plan);
+    const size_t smem = list_bytes(plan);
     // two blocks a replica when that still leaves a block to an SM and a class gives each block a round of threads
     if (N > 1 && 2 * B <= 148 && per >= 2048)
       return launch_resident_kernel(list_resident_kernel<Lat, N, ST, PER, (N > 1 ? 2 : 1)>, q, 2,
@@ -524,10 +550,7 @@ int launch_lattice_resident(const sck_plan* plan, const Common& c, int n_sweeps,
   }
   p.n_sweeps = n_sweeps;
   p.spin_bytes = (int)((resident_bytes(plan) + 15) / 16 * 16);
-  if (plan->geom.n == 1) {
-    const int floats = plan->geom.b * plan->keys;
-    if (floats <= 2048 && p.spin_bytes + 4 * floats <= (220 << 10)) p.table_floats = floats;
-  }
+  p.table_floats = table_floats(plan);
   switch (plan->resident_spec) {
     case Lat_square_1::id: return launch_lattice_resident_per<Lat_square_1>(plan, p, s);
     case Lat_triangular_1::id: return launch_lattice_resident_per<Lat_triangular_1>(plan, p, s);

@@ -180,7 +180,8 @@ class Sampler:
             L.check(L.lib().sck_plan_wait_status(self._plan, self._stream()))
 
     def path(self) -> dict:
-        """The sweep path: specialised table id (0 = generic), budget, pipeline group, resident or not."""
+        """The sweep path: specialised = 100 * kernel kind + lattice table id (0 = generic; the kinds are listed at
+        sck_plan_path in include/sck.h), budget, pipeline group, resident or not."""
         sp, bud, grp, res = ctypes.c_int32(), ctypes.c_int64(), ctypes.c_int32(), ctypes.c_int32()
         L.check(L.lib().sck_plan_path(self._plan, ctypes.byref(sp), ctypes.byref(bud), ctypes.byref(grp),
                                       ctypes.byref(res)))
