@@ -451,9 +451,16 @@ static size_t list_bytes(const sck_plan* plan) {
   return list_spin_bytes(plan) + (size_t)16 * words * plan->geom.nsite + sizeof(float) * table_floats(plan);
 }
 
-// Calls of kListSweeps sweeps and more run from neighbour lists: 16-bit slots, everything in shared memory.
+// Calls of kListSweeps sweeps and more run from neighbour lists: 16-bit slots, everything in shared memory, and no
+// class named twice. Every entry of the class list takes slots of its own, so a sweep order that repeats a class
+// (the C ABI accepts it) would need more slots than sites; it stays on lattice_resident_kernel, which walks the list.
 bool resident_lists_ok(const sck_plan* plan) {
-  return plan->resident_spec != 0 && plan->geom.nsite < 65535 && list_bytes(plan) <= kResidentSmem;
+  if (plan->resident_spec == 0 || plan->geom.nsite >= 65535 || list_bytes(plan) > kResidentSmem) return false;
+  const sck_system_desc& d = plan->desc;
+  for (int i = 0; i < d.n_classes; ++i)
+    for (int j = 0; j < i; ++j)
+      if (d.classes[i][0] == d.classes[j][0] && d.classes[i][1] == d.classes[j][1]) return false;
+  return true;
 }
 
 template <class K>

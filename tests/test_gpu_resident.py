@@ -88,3 +88,32 @@ def test_ising_class_kernel_equals_the_generic_one(name, f32, B):
         X.set_temperature(torch.linspace(1.5, 6.0, B))
         X.sweep(Y, 2)
     assert torch.equal(S, S2)
+
+
+@pytest.mark.parametrize("name", ["ising-square", "xy-triangular"])
+@pytest.mark.parametrize("order", [(0, 1, 0), (1, 1), (1,)])
+def test_repeated_and_partial_class_lists(name, order):
+    """A sweep order given through the C ABI may name a class twice or leave one out."""
+    import ctypes
+
+    from spin_colour_kernel_b200 import _lib as L
+    s = RESIDENT[name]()
+    B = 5
+    kw = dict(packed=False) if s.n == 1 else {}
+    A, G = (Sampler(s, B, device="cuda", seed=9, **kw) for _ in range(2))
+    for X in (A, G):
+        for i, k in enumerate(order):
+            X.desc.classes[i][0], X.desc.classes[i][1] = X.classes[k]
+        X.desc.n_classes = len(order)
+        h = ctypes.c_void_p()
+        L.check(L.lib().sck_plan_create(ctypes.byref(X.desc), B, X.mode, ctypes.byref(h)))
+        L.lib().sck_plan_destroy(X._plan)
+        X._plan = h
+    G.tune(False)
+    assert A.path()["specialised"] // 100 == (7 if len(set(order)) == len(order) else 6)
+    S = A.init_spins(seed=2)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(0.4, 3.0, B))
+        X.sweep(Y, 10)
+    assert torch.equal(S, S2)

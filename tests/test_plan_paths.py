@@ -75,3 +75,13 @@ def test_class_plans_name_their_kernel():
     assert plan_of(sy.ising("sc", 64), 100, L.MODE_F32).path()["specialised"] == 100 + SC
     assert plan_of(sy.heisenberg("bcc", 32), 64, L.MODE_F32).path()["specialised"] == 100 + BCC
     assert plan_of(sy.heisenberg("bcc", 32), 64, L.MODE_QUAD).path()["specialised"] == 400 + BCC
+
+
+def test_a_class_named_twice_keeps_off_the_neighbour_lists():
+    """A list takes a slot per entry of every class: with a class named twice there are more slots than sites."""
+    s = sy.ising("square", 32)
+    red, black = P.sweep_classes(s)
+    assert plan_of(s, 8, L.MODE_INT8, [red, black]).path()["specialised"] == 700 + SQUARE
+    assert plan_of(s, 8, L.MODE_INT8, [black]).path()["specialised"] == 700 + SQUARE       # a part of the sites
+    for order in ([red, black, red], [black, black]):
+        assert plan_of(s, 8, L.MODE_INT8, order).path()["specialised"] == 600 + SQUARE
