@@ -178,7 +178,9 @@ __global__ void __launch_bounds__(256, 4) ising_march_kernel(const __grid_consta
   const int row = y * g.L1 + 4 * xw;                 // this word, and those beside it, within a plane
   const int ym = (y > 0 ? y - 1 : g.L2 - 1) * g.L1 + 4 * xw, yp = (y + 1 < g.L2 ? y + 1 : 0) * g.L1 + 4 * xw;
   const int left = y * g.L1 + (xw > 0 ? 4 * xw : g.L1) - 1, right = y * g.L1 + (xw + 1 < words ? 4 * xw + 4 : 0);
-  auto word = [&](int at) { return __ldg(reinterpret_cast<const uint32_t*>(src + at)); };
+  // plain loads: a word holds bytes of the class that this launch writes, its own threads' and its neighbours', so the
+  // read-only path, which needs memory that stays as it is for the whole kernel, is not for them
+  auto word = [&](int at) { return *reinterpret_cast<const uint32_t*>(src + at); };
   // parity of the class in this row: it alternates along the walk
   int ph = CUBIC ? first_class_x(c, p.colour, 0, y, z0) : first_class_x(c, p.colour, 0, z0, 0);
   uint32_t below = spin_codes(word((z0 > 0 ? z0 - 1 : len - 1) * step + row)), here = spin_codes(word(z0 * step + row));
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(256, 4) ising_march_kernel(const __grid_consta
     const uint32_t above = spin_codes(word((z + 1 < len ? z + 1 : 0) * step + row));
     uint32_t sum = below + above;
     if constexpr (CUBIC) sum += spin_codes(word(at + ym)) + spin_codes(word(at + yp));
-    const uint32_t edge = (uint32_t)(1 + sgn(__ldg(src + at + (ph ? right : left))));
+    const uint32_t edge = (uint32_t)(1 + sgn(src[at + (ph ? right : left)]));
     const uint32_t even = here & 0x00FF00FFu, odd = (here >> 8) & 0x00FF00FFu;
     const uint32_t own = ph ? odd : even, other = ph ? even : odd;
     // neighbours along the row: the other residue's two, and one of them or the edge on the far side
