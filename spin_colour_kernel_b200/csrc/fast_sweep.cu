@@ -25,7 +25,7 @@ namespace sck {
 // instructions per attempt with one pair a thread, 75 % of the issue slots, on Heisenberg bcc 32^3 x 2). Five blocks
 // per SM: attempts/ns without a bound / at four / five / six, Heisenberg bcc J1-J2 64^3 x 2 x 64: 60 / 67 / 69 / 60;
 // XY square 512^2 x 33: 157 / 157 / 162 / 160; the quick-start case 511 / 474 / 482 / 475 us.
-template <class Lat, int N, typename ST, bool PER, int NSL>
+template <class Lat, int N, bool PER, int NSL>
 __global__ void __launch_bounds__(256, 5) spec_task_kernel(const __grid_constant__ SpecParams p) {
   follow_previous();
   const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
@@ -360,10 +360,10 @@ int find_spec(const sck_plan* p) {
 // ------------------------------------------------------------------------------------------- host: launches
 template <class Lat, int N, typename ST, bool PER, int NSL, class P>
 static void launch_one(const P& p, dim3 grid, cudaStream_t s) {
-  if constexpr (!std::is_same_v<P, SpecParams>)
+  if constexpr (std::is_same_v<P, SpecParams>)
+    launch_dependent(spec_task_kernel<Lat, N, PER, NSL>, grid, 256, s, p);
+  else
     stream_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
-  else if constexpr (N > 1)               // Ising class launches: ising_class_kernel
-    launch_dependent(spec_task_kernel<Lat, N, ST, PER, NSL>, grid, 256, s, p);
 }
 
 template <class Lat, int N, bool PER, class P>
@@ -382,10 +382,12 @@ static void launch_vec(const sck_plan* plan, const P& p, dim3 grid, cudaStream_t
 template <class Lat, bool PER, class P>
 static void launch_lat_per(const sck_plan* plan, const P& p, dim3 grid, cudaStream_t s) {
   if (plan->geom.n == 1) {
-    if (plan->mode == SCK_MODE_INT8)
-      launch_one<Lat, 1, int8_t, PER, 0>(p, grid, s);
-    else
-      launch_one<Lat, 1, float, PER, 0>(p, grid, s);
+    if constexpr (!std::is_same_v<P, SpecParams>) {      // launch_tasks refuses Ising plans
+      if (plan->mode == SCK_MODE_INT8)
+        launch_one<Lat, 1, int8_t, PER, 0>(p, grid, s);
+      else
+        launch_one<Lat, 1, float, PER, 0>(p, grid, s);
+    }
   } else if (plan->geom.n == 2) {
     launch_vec<Lat, 2, PER>(plan, p, grid, s);
   } else {
@@ -438,7 +440,9 @@ static void launch_spec_grid(const sck_plan* plan, const P& p, dim3 grid, cudaSt
 
 static int slot_replicas(const sck_plan* plan) { return seg_kernel_ok(plan) ? 1 : 2; }
 
+// Class tasks of vector models. Ising classes have kernels of their own (launch_ising_class, launch_ising_march).
 static int launch_tasks(const sck_plan* plan, SpecParams& p, cudaStream_t s) {
+  if (plan->geom.n == 1) return cuda_status(cudaErrorInvalidValue, "task launch of an Ising plan");
   int per_unit = slot_replicas(plan);
   int most = 1;
   for (int i = 0; i < p.n_tasks; ++i) {

@@ -26,3 +26,13 @@ def test_in_place_word_loads_stay_off_the_read_only_path():
     body = kernel_body("fast_sweep.cu", "ising_march_kernel")
     assert "dst[" in body and "src" in body
     assert not re.search(r"__ldg|\.nc\b|__restrict__", body)
+
+
+def test_task_launches_refuse_ising_plans():
+    """No class task kernel takes Ising spins: a task launch of an Ising plan is an error, not a launch of nothing."""
+    text = (CSRC / "fast_sweep.cu").read_text()
+    body = text[text.index("static int launch_tasks("):]
+    body = body[:body.index("\n}\n")]
+    assert re.search(r"if \(plan->geom\.n == 1\) return cuda_status\(cudaErrorInvalidValue", body)
+    one = text[text.index("static void launch_one("):]
+    assert "N > 1" not in one[:one.index("\n}\n")]
