@@ -30,11 +30,16 @@ def _cache_file() -> Path:
     return Path(root) if root else Path.home() / ".cache" / "spin_colour_kernel_b200" / "tune.json"
 
 
+# Part of every cache key: choices made among other candidates are not taken over.
+CANDIDATE_SET = 2
+
+
 def system_key(sampler) -> str:
-    """Hash of everything that shapes a sweep's work: the lowered descriptor, batch, mode and device name."""
+    """Hash of everything that shapes a sweep's work (the lowered descriptor, batch, mode and device name) and of the
+    candidate set it was tuned over."""
     import ctypes
     h = hashlib.sha256(bytes(ctypes.string_at(ctypes.addressof(sampler.desc), ctypes.sizeof(sampler.desc))))
-    h.update(f"{sampler.B}:{sampler.mode}:{torch.cuda.get_device_name(sampler.device)}".encode())
+    h.update(f"{sampler.B}:{sampler.mode}:{torch.cuda.get_device_name(sampler.device)}:{CANDIDATE_SET}".encode())
     return h.hexdigest()[:24]
 
 
@@ -111,11 +116,13 @@ def _autotune_quad(sampler, S, sweeps, use_cache, key, cache):
 
 
 def candidates(sampler):
-    """(specialised, l2_budget, resident_limit) triples worth timing for this sampler (reference layout)."""
-    out = [(0, 0, 0), (0, 0, RESIDENT_LIMIT)]
-    kind = sampler.tune(2, 0, 0)["specialised"] // 100
-    for level in range(1, kind + 1):
-        out += [(level, mb << 20, 0) for mb in CANDIDATE_BUDGETS_MB]
+    """(specialised, l2_budget, resident_limit) triples worth timing for this sampler (reference layout): generic
+    and lattice-table kernels, class by class and resident, and the L2 budgets of the class kernels, at level 2
+    where the system has segment kernels (kind 2)."""
+    out = [(0, 0, 0), (0, 0, RESIDENT_LIMIT), (1, 0, 0), (1, 0, RESIDENT_LIMIT)]
+    for level in (1, 2):
+        if sampler.tune(level, 0, 0)["specialised"] // 100 in ((1, 8) if level == 1 else (2,)):
+            out += [(level, mb << 20, 0) for mb in CANDIDATE_BUDGETS_MB]
     return out
 
 

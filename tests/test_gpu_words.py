@@ -70,3 +70,20 @@ def test_word_kernels_match_the_oracle(name, B, h, acceptance, mode):
     assert np.array_equal(M.cpu().numpy(), oob.magnetization(got))
     np.testing.assert_allclose(E2.cpu().numpy(), E.cpu().numpy(), rtol=0, atol=1e-9)
     assert torch.equal(M, M2)
+
+
+def test_autotuning_words_times_the_word_kernels(tmp_path, monkeypatch):
+    """The autotuner tells the word kernels from the generic ones, and what it applies continues the same chain."""
+    from spin_colour_kernel_b200 import autotune as at
+    monkeypatch.setenv("SCK_TUNE_CACHE", str(tmp_path / "tune.json"))
+    s = _system("sc", 0.0, "metropolis")
+    A, R = (Sampler(s, 70, device="cuda", seed=3, packed=True) for _ in range(2))
+    for X in (A, R):
+        X.set_temperature(torch.linspace(1.5, 7.0, 70))
+    S = A.init_spins(seed=4)
+    S2 = S.clone()
+    c = at.autotune(A, S, sweeps=2)
+    assert {t["specialised"] // 100 for t in c["tried"]} == {0, 5} and int(A.state[1]) == 0
+    A.sweep(S, 3)
+    R.sweep(S2, 3)
+    assert torch.equal(S, S2)

@@ -85,3 +85,24 @@ def test_a_class_named_twice_keeps_off_the_neighbour_lists():
     assert plan_of(s, 8, L.MODE_INT8, [black]).path()["specialised"] == 700 + SQUARE       # a part of the sites
     for order in ([red, black, red], [black, black]):
         assert plan_of(s, 8, L.MODE_INT8, order).path()["specialised"] == 600 + SQUARE
+
+
+@pytest.mark.parametrize("name", ["packed", "bitwise", "nanodot", "resident", "march", "vector", "open"])
+def test_autotuner_times_the_kernels_the_plan_would_run(name):
+    """Every path a plan takes untuned is among the candidates, told apart from the generic one, so tuning can not
+    leave a sampler on slower kernels than it started with."""
+    from spin_colour_kernel_b200 import autotune as at
+    A = {"packed": lambda: plan_of(sy.ising("sc", 64), 128, L.MODE_PACKED),
+         "bitwise": lambda: plan_of(sy.ising("sc", 64), 128, L.MODE_BITWISE),
+         "nanodot": lambda: plan_of(sy.nanodot(6.0, 3), 8, L.MODE_F32),
+         "resident": lambda: plan_of(sy.ising("square", 32), 32, L.MODE_INT8),
+         "march": lambda: plan_of(sy.ising("sc", 64), 100, L.MODE_INT8),
+         "vector": lambda: plan_of(sy.heisenberg("bcc", 32), 8, L.MODE_F32),      # below every budget
+         "open": lambda: plan_of(_box("sc", (70, 70, 70), per=(False,) * 3), 8, L.MODE_INT8)}[name]()
+    before = A.path()
+    paths = [A.tune(*c) for c in at.candidates(A)]
+    assert before in paths
+    assert (before["specialised"] > 0) and any(p["specialised"] == 0 for p in paths)
+    sig = {(p["specialised"], p["group"], p["resident"]) for p in paths}          # what the autotuner tells apart
+    assert len(sig) >= 2
+    A.tune(*at.candidates(A)[0])
