@@ -486,7 +486,15 @@ static void launch_ising_t(const sck_plan* plan, const IsingClassParams& p, dim3
   }
 }
 
-// The marching kernel's systems: the walk and both row directions alternate between the two colours.
+// The marching kernel's systems: the walk and both row directions alternate between the two colours, the words of a
+// plane or row fill at least 7/16 of its blocks' threads, and there are enough walks of eight sites to occupy the GPU.
+// Everything else takes ising_class_kernel. Class kernel against marching, us a sweep:
+//   filled:  square 4 x 60,000 x 100 (1 word of 256) 129 / 4,425; 256 x 1,024 x 33 (64) 50.2 / 57.8;
+//            500^2 x 33 (125) 48.6 / 45.4; 1,024 x 256 x 33 (256) 50.2 / 44.6
+//   walks:   sc 64^3 x 1 (8,192) 7.6 / 14.0, x 3 (24,576) 14.7 / 15.1, x 4 (32,768) 18.1 / 15.2; sc 96^3 x 1 (27,648)
+//            15.8 / 14.4; square 512^2 x 3 (24,576) 13.4 / 13.6, x 4 (32,768) 16.4 / 13.9
+constexpr long long kMarchWalks = 26000;
+
 bool ising_march_plan(const sck_plan* plan) {
   const Geometry& g = plan->geom;
   if (plan->mode != SCK_MODE_INT8 || g.has_mask || g.L1 % 4 != 0 || !spec_periodic_box(plan)) return false;
@@ -495,7 +503,9 @@ bool ising_march_plan(const sck_plan* plan) {
   if (col.r != 1 || col.m[0] != 2) return false;
   for (int k = 0; k < g.dim; ++k)
     if (col.K[0][k] != 1) return false;
-  return true;
+  const int cols = g.L1 / 4 * (g.dim == 3 ? g.L2 : 1), len = g.dim == 3 ? g.L3 : g.L2;
+  if (16 * (long long)cols < 7 * 256 * (long long)((cols + 255) / 256)) return false;
+  return (long long)cols * ((len + 7) / 8) * plan->Bp >= kMarchWalks;
 }
 
 // Its 4-byte loads need spins that start on 4 bytes.

@@ -117,3 +117,33 @@ def test_repeated_and_partial_class_lists(name, order):
         X.set_temperature(torch.linspace(0.4, 3.0, B))
         X.sweep(Y, 10)
     assert torch.equal(S, S2)
+
+
+# boxes and replica counts the marching kernel takes: rows of words at half a block, over one block, nearly full
+# blocks; walks with a remainder, of one chunk, and two layers thick
+MARCHING = {
+    "square": (lambda: _sys(1, "square", (512, 20), h=(0.2,)), 70),
+    "square-wide": (lambda: _sys(1, "square", (1040, 10), acceptance="barker"), 60),
+    "square-long": (lambda: _sys(1, "square", (448, 270)), 7),
+    "sc": (lambda: _sys(1, "sc", (16, 32, 18)), 71),
+    "sc-blocks": (lambda: _sys(1, "sc", (64, 34, 20), J={1: -1.0}, acceptance="barker"), 33),
+    "sc-thin": (lambda: _sys(1, "sc", (4, 112, 2), h=(-0.4,)), 240),
+}
+
+
+@pytest.mark.parametrize("name", sorted(MARCHING))
+@pytest.mark.parametrize("values", ["spins", "any"])
+def test_marching_kernel_equals_the_generic_one(name, values):
+    build, B = MARCHING[name]
+    s = build()
+    A, G = (Sampler(s, B, device="cuda", seed=3, packed=False) for _ in range(2))
+    assert A.tune(True, 0, 0)["specialised"] // 100 == 8
+    G.tune(False, 0, 0)
+    S = A.init_spins(seed=2)
+    if values == "any":              # any value counts by its sign; a zero spin stays zero
+        S = torch.randint(-127, 128, S.shape, generator=torch.Generator().manual_seed(1)).to(S)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(1.5, 6.0, B))
+        X.sweep(Y, 3)
+    assert torch.equal(S, S2)
