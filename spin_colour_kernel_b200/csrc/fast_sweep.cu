@@ -361,7 +361,7 @@ int find_spec(const sck_plan* p) {
 template <class Lat, int N, typename ST, bool PER, int NSL, class P>
 static void launch_one(const P& p, dim3 grid, cudaStream_t s) {
   if constexpr (std::is_same_v<P, SpecParams>)
-    launch_dependent(spec_task_kernel<Lat, N, PER, NSL>, grid, 256, s, p);
+    launch_dependent(spec_task_kernel<Lat, N, PER, NSL>, grid, 256, 5, s, p);
   else
     stream_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
 }

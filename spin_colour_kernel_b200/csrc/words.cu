@@ -504,9 +504,9 @@ int launch_word_columns(const sck_plan* plan, const ObsParams& p, cudaStream_t s
 // --------------------------------------------------------------------------------------------- host side
 template <class Lat, bool BARKER>
 static void launch_packed(const WordParams& p, int parts, dim3 grid, cudaStream_t s) {
-  if (parts == 1) launch_dependent(packed_lattice_kernel<Lat, 32, BARKER>, grid, 256, s, p);
-  else if (parts == 2) launch_dependent(packed_lattice_kernel<Lat, 16, BARKER>, grid, 256, s, p);
-  else launch_dependent(packed_lattice_kernel<Lat, 8, BARKER>, grid, 256, s, p);
+  if (parts == 1) launch_dependent(packed_lattice_kernel<Lat, 32, BARKER>, grid, 256, 4, s, p);
+  else if (parts == 2) launch_dependent(packed_lattice_kernel<Lat, 16, BARKER>, grid, 256, 4, s, p);
+  else launch_dependent(packed_lattice_kernel<Lat, 8, BARKER>, grid, 256, 4, s, p);
 }
 
 template <class Lat>
@@ -515,11 +515,11 @@ static void launch_word_t(const sck_plan* plan, const WordParams& p, int parts, 
     if (plan->geom.acceptance == SCK_BARKER) launch_packed<Lat, true>(p, parts, grid, s);
     else launch_packed<Lat, false>(p, parts, grid, s);
   } else if (plan->mode == SCK_MODE_BITWISE) {
-    if (p.c.field) launch_dependent(bitwise_shared_lattice_kernel<Lat, true>, grid, 256, s, p);
-    else launch_dependent(bitwise_shared_lattice_kernel<Lat, false>, grid, 256, s, p);
+    if (p.c.field) launch_dependent(bitwise_shared_lattice_kernel<Lat, true>, grid, 256, 5, s, p);
+    else launch_dependent(bitwise_shared_lattice_kernel<Lat, false>, grid, 256, 5, s, p);
   } else {
-    if (p.c.field) launch_dependent(bitwise_independent_lattice_kernel<Lat, true>, grid, 256, s, p);
-    else launch_dependent(bitwise_independent_lattice_kernel<Lat, false>, grid, 256, s, p);
+    if (p.c.field) launch_dependent(bitwise_independent_lattice_kernel<Lat, true>, grid, 256, 4, s, p);
+    else launch_dependent(bitwise_independent_lattice_kernel<Lat, false>, grid, 256, 4, s, p);
   }
 }
 

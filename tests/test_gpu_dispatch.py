@@ -1,0 +1,77 @@
+"""Kernel variants that only larger launches, odd tails or certain sizes select, each against a path of its own: the
+generic kernels (bit for bit where the arithmetic is shared), the interleaved layout, the systems of a batch swept on
+their own, or the oracle. Sizes are the smallest that reach the variant, given beside each case."""
+
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import cases as C
+from oracle import observables as oob
+from spin_colour_kernel_b200 import _lib as L
+from spin_colour_kernel_b200 import crystals as cr
+from spin_colour_kernel_b200 import system as sy
+from spin_colour_kernel_b200.sampler import Sampler, SamplerBatch
+
+pytestmark = pytest.mark.gpu
+
+
+def _sys(n, crystal, box, **kw):
+    c = cr.make(crystal)
+    return sy.System(f"{crystal} n={n}", n, c, box, (True,) * c.D, {1: 1.0}, **kw)
+
+
+def _words(A, seed):
+    """Random words: every replica's spins +-1 with equal probability."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    shape = (A.W, 1) + A.sys.shape
+    return torch.randint(-2 ** 31, 2 ** 31, shape, generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+
+
+def _word_temperatures(B):
+    W = -(-B // 32)
+    return torch.linspace(1.5, 7.0, W).repeat_interleave(32)[:B]
+
+
+# Class launches of 64, 512 and 768 blocks (alone on half the SMs; too few to overlap; overlapping), captured: a replay
+# continues the chain of plain calls.
+DEPENDENT = {
+    "vector-64": (lambda: _sys(2, "square", (180, 180)), 2, {}),
+    "vector-512": (lambda: _sys(2, "square", (180, 180)), 16, {}),
+    "vector-768": (lambda: _sys(2, "square", (180, 180)), 24, {}),
+    "heisenberg": (lambda: sy.heisenberg("bcc", 24), 33, {}),
+    "int8": (lambda: _sys(1, "triangular", (300, 300)), 5, dict(packed=False)),
+    "packed": (lambda: _sys(1, "sc", (32, 32, 32)), 70, dict(packed=True)),
+    "bitwise": (lambda: _sys(1, "sc", (32, 32, 32)), 70, dict(bitwise=True)),
+    "independent": (lambda: _sys(1, "triangular", (60, 60)), 70, dict(bitwise=True, independent=True)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(DEPENDENT))
+def test_captured_class_launches_continue_the_chain(name):
+    build, B, kw = DEPENDENT[name]
+    s = build()
+    A, R = (Sampler(s, B, device="cuda", seed=8, **kw) for _ in range(2))
+    for X in (A, R):
+        X.tune(True, 0, 0)
+        X.set_temperature(_word_temperatures(B) if X.bitwise else torch.linspace(0.5, 4.0, B))
+    S = A.init_spins(seed=2)
+    S2 = S.clone()
+    replay = A.graph(S, 3)                     # one sweep before the capture
+    for _ in range(2):
+        replay()
+    R.sweep(S2, 7)
+    torch.cuda.synchronize()
+    assert int(A.state[1]) == int(R.state[1]) == 7
+    assert torch.equal(S, S2)
+    if s.n == 1:                               # and the generic kernels', which launch without overlap
+        G = Sampler(s, B, device="cuda", seed=8, **kw)
+        G.tune(False, 0, 0)
+        G.set_temperature(_word_temperatures(B) if G.bitwise else torch.linspace(0.5, 4.0, B))
+        S3 = G.init_spins(seed=2)
+        G.sweep(S3, 7)
+        assert torch.equal(S, S3)
