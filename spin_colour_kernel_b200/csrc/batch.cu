@@ -39,7 +39,33 @@ constexpr int kBatchMaxSystems = 256;
 // neighbours' offsets once for all of them. Two sweeps of 24 XY systems (40 M attempts): one pair and eight passes
 // 603 us, four pairs and two passes 515; smaller items 592 (half), 781 (a quarter), larger 498 (twice, but fewer
 // items than blocks for small batches).
+//
+// A class of fewer than eight runs does not fill an item: more pairs then mean a longer item and fewer of them, which
+// pays only when the blocks have more items than they can take at once. item_groups therefore gives a system several
+// pairs when its items grow no longer than the batch's longest or by no more than an eighth, when they grow by no more than
+// a third and a class step holds items for most SMs (96), or when it holds twice the resident blocks (1,184). Systems
+// outside the tables form every site anew for each replica and gain from full items alone. Two sweeps, one pair / four pairs:
+//   XY square 24^2 x 8, one system 24.8 / 42.3 us; 40^2 x 32, one 36.9 / 51.5, 64 of them x 32 143 / 105;
+//   54^2 x 16, one 47 / 51, eight (128 items) 73.7 / 60.8; triangular 72^2 x 8, 16 systems 136 / 115;
+//   Heisenberg bcc 12^3 x 8 250 / 285, 24^3 x 8, four systems 575 / 522
 constexpr int kBatchItemPasses = 8;
+
+// Replica pairs (vector models) or replicas (Ising) per streaming item of a system whose class takes `runs` runs of 256
+// sites, of `slots` pairs or replicas; `longest`: runs of the batch's longest item; `items`: items of a class step of
+// the whole batch with one pair each.
+static int item_groups(long long runs, long long slots, long long longest, long long items, bool table) {
+  int groups = 1;
+  while (groups < 4 && 2 * groups <= slots) {
+    const long long length = std::min<long long>(kBatchItemPasses, 2 * groups * runs);
+    const bool full = runs >= kBatchItemPasses;
+    const bool ok = table ? length <= longest || 7 * length <= 8 * runs || (3 * length <= 4 * runs && items >= 96) ||
+                                items >= 2 * 592
+                          : full && items >= 96;
+    if (!ok) break;
+    groups *= 2;
+  }
+  return groups;
+}
 constexpr int kBatchMaxClasses = 32;
 
 struct SysDev {
@@ -450,6 +476,17 @@ int sck_batch_bind(sck_batch* b, const sck_buffers* buffers, void* workspace, vo
   int* res_off = (int*)(img + b->layout.res_off);
   long long res_total = 0;
   std::vector<long long> step_total(b->max_classes, 0);
+  auto unit_of = [](const sck_plan* plan) { return plan->geom.n == 1 ? 1 : 2; };
+  auto runs_of = [](const sck_plan* plan) {
+    return ((long long)plan->geom.L2 * plan->geom.L3 * plan->bx + 255) / 256;
+  };
+  long long longest = 1, one_pair_items = 0;
+  for (int s = 0; s < b->n; ++s) {
+    if (b->resident[s]) continue;
+    const long long runs = runs_of(b->plans[s]), unit = unit_of(b->plans[s]);
+    longest = std::max(longest, std::min<long long>(runs, kBatchItemPasses));
+    one_pair_items += (runs + kBatchItemPasses - 1) / kBatchItemPasses * ((b->plans[s]->Bp + unit - 1) / unit);
+  }
   for (int s = 0; s < b->n; ++s) {
     const sck_plan* plan = b->plans[s];
     const sck_buffers& bu = buffers[s];
@@ -469,14 +506,13 @@ int sck_batch_bind(sck_batch* b, const sck_buffers* buffers, void* workspace, vo
     }
     d.resident = b->resident[s];
     const long long per = (long long)d.c.rows * d.c.bx;
-    const int unit = plan->geom.n == 1 ? 1 : 2;
-    int groups = 1;
-    while (groups < 4 && 2 * groups * unit <= plan->Bp) groups *= 2;
+    const bool table = plan->spec == Lat_square_1::id || plan->spec == Lat_triangular_1::id ||
+                       plan->spec == Lat_sc_1::id;
+    const int unit = unit_of(plan);
+    const int groups = item_groups(runs_of(plan), plan->Bp / unit, longest, one_pair_items, table);
     d.rpi = groups * unit;
     d.passes = kBatchItemPasses / groups;
     d.chunks = (int)((per + 256 * d.passes - 1) / (256 * d.passes));
-    const bool table = plan->spec == Lat_square_1::id || plan->spec == Lat_triangular_1::id ||
-                       plan->spec == Lat_sc_1::id;
     d.spec = table ? plan->spec : 0;
     d.per = table ? spec_periodic_box(plan) : 0;
     for (int a = 0; a < SCK_MAX_BASIS; ++a)

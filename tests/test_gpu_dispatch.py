@@ -75,3 +75,43 @@ def test_captured_class_launches_continue_the_chain(name):
         S3 = G.init_spins(seed=2)
         G.sweep(S3, 7)
         assert torch.equal(S, S3)
+
+
+def _batch(systems, B):
+    A, R = ([Sampler(s, B, device="cuda", seed=20 + i) for i, s in enumerate(systems)] for _ in range(2))
+    for X in A + R:
+        X.set_temperature(torch.linspace(0.4, 1.6, B))
+    S = [X.init_spins(seed=i) for i, X in enumerate(A)]
+    return A, R, S, [x.clone() for x in S]
+
+
+# Streaming items of several replica pairs: classes that fill their items (64^2 and up), shorter ones beside them, and
+# replica counts that leave an item with one replica, with three, and with a pair.
+@pytest.mark.parametrize("B", [9, 11, 18])
+def test_batch_items_of_several_pairs(B):
+    systems = [_sys(2, "square", (64, 64)), _sys(2, "triangular", (90, 84)), _sys(2, "sc", (18, 16, 20)),
+               _sys(2, "square", (24, 20)), sy.xy("square", 100)]
+    A, R, S, S2 = _batch(systems, B)
+    b = SamplerBatch(A, S, resident_limit=0)
+    b.sweep(3)
+    b.check_waits()
+    for X, Y, Z in zip(R, S2, S):
+        C.batch_twin_tune(X, 0)
+        X.sweep(Y, 3)
+        assert torch.equal(Y, Z), X.sys.name
+
+
+# Items per class of one system alone: a class that fills items shares them out among four pairs, one that does not keeps
+# an item per pair (256 sites: 1 run), unless its items grow by at most an eighth (1,728 sites: 7 runs) or items abound.
+@pytest.mark.parametrize("box,systems,B,items", [((16, 16), 8, 8, 4), ((24, 24), 1, 32, 16), ((64, 64), 1, 32, 16),
+                                                 ((16, 16), 80, 32, 4), ((58, 58), 1, 32, 16)])
+def test_batch_items_follow_the_length_of_a_class(box, systems, B, items):
+    ss = [_sys(2, "square", box) for _ in range(systems)]
+    A, R, S, S2 = _batch(ss, B)
+    b = SamplerBatch(A, S, resident_limit=0)
+    assert b.info()["step_blocks"] == 2 * systems * items
+    b.sweep(2)
+    X, Y = R[-1], S2[-1]
+    C.batch_twin_tune(X, 0)
+    X.sweep(Y, 2)
+    assert torch.equal(Y, S[-1])
