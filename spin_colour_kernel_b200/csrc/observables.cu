@@ -631,9 +631,19 @@ __device__ __forceinline__ double solid_angle(const double (&a)[3], const double
   return 2.0 * atan2(num, den);
 }
 
-// A block's time is its longest thread's chain of FP64 arctangents, so a layer spreads over 1,024 threads, and the sum
-// is a tree (one thread adding 256 partials in turn: 14 us for 64 layers of 39 x 39).
+// A block's time is its longest thread's chain of FP64 arctangents, so a layer spreads over as many threads as have a
+// plaquette each while blocks have SMs to themselves, and the sum is a tree (one thread adding 256 partials in turn: 14
+// us for 64 layers of 39 x 39). With several blocks to an SM the FP64 pipe is busy anyway, and smaller blocks pack
+// better. us at 256 / 512 / 1,024 threads: 39 x 39 plaquettes, 64 replicas 9.4 / 6.4 / 5.9, 200: 10.6 / 9.1 / 10.4,
+// 600: 20.5 / 19.4 / 24.1, 1,000: 26.7 / 26.7 / 34.1; 15 x 15, 1,000 replicas: 5.8 / 9.0 / 15.0.
 constexpr int kChargeThreads = 1024;
+
+static int charge_threads(const Geometry& g, int batch) {
+  const int plaquettes = (g.L1 - 1) * (g.L2 - 1);
+  int t = batch <= 148 ? kChargeThreads : (batch <= 6 * 148 ? 512 : 256);
+  while (t > 256 && t / 2 >= plaquettes) t /= 2;
+  return t;
+}
 
 __global__ void __launch_bounds__(kChargeThreads) topological_charge_kernel(const float* __restrict__ spins,
                                                                  const int8_t* __restrict__ mask, Geometry g, int z,
@@ -664,15 +674,15 @@ __global__ void __launch_bounds__(kChargeThreads) topological_charge_kernel(cons
   __syncthreads();
   if (threadIdx.x == 0) {
     double sum = 0.0;
-#pragma unroll
-    for (int i = 0; i < kChargeThreads / 32; ++i) sum += part[i];
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) sum += part[i];
     Q[rep] = sum / (4.0 * 3.14159265358979323846);
   }
 }
 
 int launch_topological_charge(const sck_plan* plan, const float* spins, const int8_t* mask, int batch, int z,
                               double* Q, cudaStream_t s) {
-  topological_charge_kernel<<<batch, kChargeThreads, 0, s>>>(spins, plan->geom.has_mask ? mask : nullptr, plan->geom, z, Q);
+  topological_charge_kernel<<<batch, charge_threads(plan->geom, batch), 0, s>>>(
+      spins, plan->geom.has_mask ? mask : nullptr, plan->geom, z, Q);
   return cuda_status(cudaGetLastError(), "topological charge");
 }
 

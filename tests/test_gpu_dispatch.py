@@ -115,3 +115,19 @@ def test_batch_items_follow_the_length_of_a_class(box, systems, B, items):
     C.batch_twin_tune(X, 0)
     X.sweep(Y, 2)
     assert torch.equal(Y, S[-1])
+
+
+@pytest.mark.parametrize("Rd,layers,B", [(6.0, 3, 200), (10.0, 3, 150), (18.3, 5, 148), (18.3, 5, 200), (18.3, 5, 900)])
+def test_topological_charge_of_any_block_size(Rd, layers, B):
+    """Blocks of 256, 512 and 1,024 threads give the charges that single replicas (as many threads as a layer has
+    plaquettes, at most 1,024) give, up to the order of an FP64 sum of at most 3,000 terms below 4 pi."""
+    s = sy.nanodot(Rd=Rd, L=layers)
+    A, R = Sampler(s, B, device="cuda", seed=1), Sampler(s, 1, device="cuda", seed=1)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn((B, 3) + s.shape, generator=g, device="cuda")
+    x = (x / x.norm(dim=1, keepdim=True) * torch.as_tensor(s.site_mask(), device="cuda")).contiguous()
+    Q = A.topological_charge(x, 1)
+    for r in (0, B // 2, B - 1):
+        q = R.topological_charge(x[r:r + 1].contiguous(), 1)
+        assert abs(float(Q[r]) - float(q[0])) < 3000 * 4 * np.pi * 2.0 ** -52
+    assert float(Q.abs().max()) > 0
