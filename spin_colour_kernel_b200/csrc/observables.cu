@@ -551,8 +551,13 @@ static int obs_blocks_words(const sck_plan* plan, int batch) {
   return want < per_rep ? (want < 1 ? 1 : want) : per_rep;
 }
 
-static bool obs_columns(const sck_plan* plan, int storage) {
-  return storage == SCK_MODE_PACKED && plan->word_spec != 0 && word_columns_ok(plan);
+// A column's chain of sites and its transposes cost the four-sublattice fcc cell 11 us however small the box, so few
+// words of a small one stay with the generic kernel: us generic / columns, 6^3 x 128 replicas (3,456 words) 10.6 / 10.8,
+// 8^3 x 64 (4,096) 10.5 / 11.9, 8^3 x 128 (8,192) 15.7 / 12.0, 10^3 x 64 (8,000) 17.1 / 11.9. The other tables gain at
+// every size measured (square 8^2 x 32: 5.0 / 4.5; bcc 6^3 x 32: 6.4 / 6.0).
+static bool obs_columns(const sck_plan* plan, int storage, int batch) {
+  if (storage != SCK_MODE_PACKED || plan->word_spec == 0 || !word_columns_ok(plan)) return false;
+  return plan->word_spec != Lat_fcc_1::id || (long long)plan->geom.nsite * ((batch + 31) / 32) > 4096;
 }
 
 // Slots per replica a call without a workspace is accepted by: the launch's own count, except that the column
@@ -565,7 +570,7 @@ static int obs_scratch_slots(const sck_plan* plan, int storage, int batch) {
 
 int obs_launch_blocks(const sck_plan* plan, int storage, int batch) {
   if (storage == SCK_MODE_QUAD) return quad_obs_blocks(plan);
-  if (obs_columns(plan, storage)) return word_column_blocks(plan, batch);
+  if (obs_columns(plan, storage, batch)) return word_column_blocks(plan, batch);
   return obs_scratch_slots(plan, storage, batch);
 }
 
@@ -803,7 +808,7 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
   // float32 storage of a tiled-geometry system with its lattice table on: bands of OBS_TY rows
   const bool tile = obs_tiled(plan, storage);
   p.blocks_per_rep = obs_launch_blocks(plan, storage, batch);
-  if (scratch_blocks > 0 && p.blocks_per_rep > scratch_blocks && obs_columns(plan, storage))
+  if (scratch_blocks > 0 && p.blocks_per_rep > scratch_blocks && obs_columns(plan, storage, batch))
     p.blocks_per_rep = scratch_blocks;
   p.fd_plane = make_fastdiv((uint32_t)plan->geom.plane);
   p.fd_L1 = make_fastdiv((uint32_t)plan->geom.L1);
@@ -846,7 +851,7 @@ int launch_observables(const sck_plan* plan, const void* spins, int storage, int
       case Lat_bcc_1_2::id: launch_obs_extra<Lat_bcc_1_2>(p, grid, s); break;
       default: launch_obs_extra<Lat_fcc_1>(p, grid, s); break;
     }
-  } else if (obs_columns(plan, storage)) {
+  } else if (obs_columns(plan, storage, batch)) {
     const int rc = launch_word_columns(plan, p, s);
     if (rc != SCK_OK) return rc;
   } else if (p.storage == 2 && obs_words_ok(plan, storage)) {

@@ -37,6 +37,18 @@ def _word_temperatures(B):
     return torch.linspace(1.5, 7.0, W).repeat_interleave(32)[:B]
 
 
+@pytest.mark.parametrize("B", [33, 160])
+def test_fcc_word_observables_on_both_kernels(B):
+    """840 sites: two words stay on the generic kernel, five take the columns."""
+    s = _sys(1, "fcc", (6, 5, 7), h=(0.1,))
+    A = Sampler(s, B, device="cuda", seed=2, packed=True)
+    S = A.init_spins(seed=3)
+    E, M = A.observables(S)
+    x = A.unpack(S).cpu().numpy()
+    np.testing.assert_allclose(E.cpu().numpy(), oob.energy(s, x), rtol=0, atol=1e-9)
+    assert np.array_equal(M.cpu().numpy(), oob.magnetization(x))
+
+
 # Class launches of 64, 512 and 768 blocks (alone on half the SMs; too few to overlap; overlapping), captured: a replay
 # continues the chain of plain calls.
 DEPENDENT = {
