@@ -287,3 +287,21 @@ def test_trained_network_decorrelates_faster_than_untrained():
     t_, u_ = out["trained"], out["untrained"]
     assert t_["acceptance"] > 0.3 and t_["acceptance"] > 50 * u_["acceptance"], out
     assert t_["tau_E"] < 0.95 * u_["tau_E"] and t_["tau_M"] < u_["tau_M"], out
+
+
+@pytest.mark.parametrize("rows", [12160, 12288, 12416])
+def test_forward_of_large_batches_equals_that_of_small_ones(rows):
+    """From 12,288 rows on a block multiplies all columns of a hidden layer: rows at both ends of the batch against the
+    same rows alone (equal up to FP32 summation order and a rare bfloat16 rounding tie of an activation)."""
+    _need_gpu()
+    from spin_colour_kernel_b200.learned import BlockProposal
+    P = BlockProposal(16, 1, groups=16, params=_random_params(15))
+    b, x = _inputs(rows, 16)
+    X = _to_dev(b, x)
+    big, lq = P.forward(X)
+    P.check_waits()
+    for part in (slice(0, 256), slice(rows - 256, rows)):
+        small, lq2 = P.forward(X[part].contiguous())
+        d = (big[part] - small).abs()
+        assert float(d.median()) < 1e-5 and float(d.max()) < 0.05
+        assert float((lq[part] - lq2).abs().max()) < 0.1
