@@ -37,6 +37,63 @@ def _word_temperatures(B):
     return torch.linspace(1.5, 7.0, W).repeat_interleave(32)[:B]
 
 
+# A block of the packed kernel takes a whole word where class blocks x words reach 592, half a word from 296: boxes of
+# 384 (sc), 300 (bcc) and 188 (fcc) blocks a class, the last word full, partial, and partial in a single word; counts
+# of six neighbours (own spin in the fourth plane) and of eight and twelve.
+@pytest.mark.parametrize("crystal,box,B", [("sc", (64, 64, 48), 50), ("sc", (64, 64, 48), 20), ("bcc", (80, 80, 12), 64),
+                                           ("bcc", (80, 80, 12), 31), ("fcc", (40, 40, 30), 101), ("fcc", (40, 40, 30), 50)])
+@pytest.mark.parametrize("acceptance", ["metropolis", "barker"])
+def test_packed_words_by_whole_and_half_words(crystal, box, B, acceptance):
+    s = _sys(1, crystal, box, h=(0.2,) if B % 2 else None, acceptance=acceptance)
+    A, G = (Sampler(s, B, device="cuda", seed=17, packed=True) for _ in range(2))
+    G.tune(False)
+    S = _words(A, 3)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(1.5, 7.0, B))
+        X.sweep(Y, 2)
+    assert torch.equal(S, S2)
+
+
+# Several units (groups of four words, or words) a block: 384 blocks a class leave 4 grid rows for 5 groups or 19 words.
+@pytest.mark.parametrize("independent", [False, True])
+@pytest.mark.parametrize("h,acceptance", [(0.0, "metropolis"), (0.1, "metropolis"), (0.1, "barker")])
+def test_bitwise_words_with_several_units_a_block(independent, h, acceptance):
+    B = 600
+    s = _sys(1, "sc", (64, 64, 48), h=(h,) if h else None, acceptance=acceptance)
+    A, G = (Sampler(s, B, device="cuda", seed=5, bitwise=True, independent=independent) for _ in range(2))
+    G.tune(False)
+    S = _words(A, 4)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(_word_temperatures(B))
+        X.sweep(Y, 2)
+    assert torch.equal(S, S2)
+
+
+def test_column_observables_with_fewer_blocks_than_items():
+    """24 items a word for 19 blocks, and for the 4 that the scratch of the call without a workspace holds."""
+    B = 4096
+    s = _sys(1, "bcc", (64, 48, 9), h=(0.3,))
+    A = Sampler(s, B, device="cuda", seed=1, packed=True)
+    S = _words(A, 6)
+    buf = A._buffers(S)
+
+    def call(fn, *ws):
+        E = torch.full((B,), np.nan, dtype=torch.float64, device="cuda")
+        M = torch.full((B, s.b, 1), np.nan, dtype=torch.float64, device="cuda")
+        L.check(fn(A._plan, ctypes.byref(buf), S.data_ptr(), L.MODE_PACKED, B, E.data_ptr(), M.data_ptr(), *ws, A._stream()))
+        return E, M
+    lib = L.lib()
+    E1, M1 = call(lib.sck_observables, A._workspace(B).data_ptr())
+    E2, M2 = call(lib.sck_observables_noalloc)
+    A.tune(False)
+    E3, M3 = call(lib.sck_observables, A._workspace(B).data_ptr())
+    for E, M in ((E2, M2), (E3, M3)):          # sums of +-1 and +-J: exact but for the field's rounding
+        torch.testing.assert_close(E, E1, rtol=0, atol=1e-8)
+        assert torch.equal(M, M1)
+
+
 @pytest.mark.parametrize("B", [33, 160])
 def test_fcc_word_observables_on_both_kernels(B):
     """840 sites: two words stay on the generic kernel, five take the columns."""
@@ -87,6 +144,44 @@ def test_captured_class_launches_continue_the_chain(name):
         S3 = G.init_spins(seed=2)
         G.sweep(S3, 7)
         assert torch.equal(S, S3)
+
+
+# States just above 96 MB, whose interleaved class launches prefetch the rows of later blocks: the cubic tiles, rows of
+# two residues and of one, with a last quad that is not full; in the reference layout, units of four replica pairs with a
+# remainder.
+@pytest.mark.parametrize("n,crystal,box,B", [(3, "sc", (64, 64, 64), 35), (3, "bcc", (33, 34, 35), 105),
+                                             (2, "square", (512, 512), 49), (3, "sc", (62, 60, 58), 37)])
+def test_prefetching_interleaved_launches_and_pair_units_agree(n, crystal, box, B):
+    s = _sys(n, crystal, box)
+    Q, R = (Sampler(s, B, device="cuda", seed=4, layout=layout) for layout in ("quad", "reference"))
+    R.tune(True, 0, 0)
+    assert -(-B // 4) * 16 * n * s.nsite > 96 << 20
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn((B, n) + s.shape, generator=g, device="cuda")
+    x /= x.norm(dim=1, keepdim=True)
+    X = Q.pack(x)
+    for A, Y in ((Q, X), (R, x)):
+        A.set_temperature(torch.linspace(0.5, 2.5, B))
+        A.sweep(Y, 2)
+    assert torch.equal(Q.unpack(X), x)
+
+
+# Replicas a thread of the int8 / float32 class kernel keeps: two at 41 replicas of 118 blocks, eight at 163; the last
+# thread row has one and three.
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("B", [41, 163])
+def test_ising_class_kernel_with_an_odd_tail_of_replicas(f32, B):
+    s = _sys(1, "triangular", (300, 300), h=(0.1,))
+    kw = dict(packed=False, spin_dtype=torch.float32 if f32 else torch.int8)
+    A, G = (Sampler(s, B, device="cuda", seed=6, **kw) for _ in range(2))
+    assert A.tune(True, 0, 0)["specialised"] // 100 == 1
+    G.tune(False, 0, 0)
+    S = A.init_spins(seed=2)
+    S2 = S.clone()
+    for X, Y in ((A, S), (G, S2)):
+        X.set_temperature(torch.linspace(1.0, 5.0, B))
+        X.sweep(Y, 2)
+    assert torch.equal(S, S2)
 
 
 def _batch(systems, B):

@@ -289,6 +289,26 @@ def test_trained_network_decorrelates_faster_than_untrained():
     assert t_["tau_E"] < 0.95 * u_["tau_E"] and t_["tau_M"] < u_["tau_M"], out
 
 
+# 64 rows: one chunk; 832: chunks of 320, 320 and 192 rows, and forward layers outside the tcgen05 tiles; 8,256: 26
+# chunks of at most 32, the last of 256
+@pytest.mark.parametrize("rows", [64, 832, 8256])
+def test_gradients_of_uneven_chunks_match_oracle(rows):
+    _need_gpu()
+    from spin_colour_kernel_b200.learned import BlockProposal
+    params = _random_params(13)
+    P = BlockProposal(16, 1, groups=16, params=params)
+    b, x = _inputs(rows, 14)
+    loss, grads = P.grads(_to_dev(b, x))
+    mk = MD.masks(96, 64, 256, groups=16)
+    ref_loss, ref = MD.loss_and_grads(params, mk, b, x)
+    assert abs(loss - ref_loss) < 1e-3 * max(1.0, abs(ref_loss))
+    for li, ((dW, db), (rW, rb)) in enumerate(zip(grads, ref)):
+        rel_w = np.linalg.norm(dW - rW) / np.linalg.norm(rW)
+        rel_b = np.linalg.norm(db - rb) / max(np.linalg.norm(rb), 1e-12)
+        assert rel_w < 3e-2 and rel_b < 3e-2, (li, rel_w, rel_b)
+        assert np.all(dW[mk[li] == 0] == 0)
+
+
 @pytest.mark.parametrize("rows", [12160, 12288, 12416])
 def test_forward_of_large_batches_equals_that_of_small_ones(rows):
     """From 12,288 rows on a block multiplies all columns of a hidden layer: rows at both ends of the batch against the
