@@ -152,17 +152,28 @@ static int quad_blocks_x(const sck_plan* plan) {
 // 64^3 x 2 x 1,536 in us: 10,530 without, 9,900 / 9,710 / 9,900 / 9,880 at 40 / 80 / 120 / 200 ahead, 10,160 at 450,
 // 13,600 at 900 (rows fall out of L2 before they are used). 48^3 x 2: 170 MB 65.7 -> 71.2 attempts/ns, 127 MB
 // 62.9 -> 65.9, 85 MB 64.4 -> 64.0.
-constexpr unsigned kPrefetchBlocks = 100;
-constexpr size_t kPrefetchState = (size_t)96 << 20;
+//
+// On the compile-time cube of the four-class lattices (bcc J1-J2 and fcc, 64^3) 100 blocks are too far ahead, and states
+// of up to twice L2 do better without: one sweep of J1-J2 in us, without / 40 / 100 ahead, 126 MB 149 / 159 / 158, 277 MB
+// 301 / 306 / 320, 403 MB 425 / 419 / 460, 805 MB 829 / 746 / 880, 1.6 GB 1,647 / 1,454 / 1,590, 9.7 GB 10,075 / 9,852 /
+// 9,794; fcc 201 MB 198 / 203 / 212, 302 MB 294 / 279 / 305, 805 MB 733 / 657 / 730. The other lattices at 64^3 gain from
+// 100 MB on at either distance (sc 138 MB 100.9 / 85.7 / 83.4, bcc 201 MB 131 / 118 / 125), as do other boxes of
+// these (J1-J2 48^3 149 MB 189 / 176 / 170, 80^3 147 MB 185 / - / 171).
+constexpr unsigned kPrefetchBlocks = 100, kPrefetchBlocksCube = 40;
+constexpr size_t kPrefetchState = (size_t)96 << 20, kPrefetchStateCube = (size_t)272 << 20;
 
 static int launch_quad_params(const sck_plan* plan, QuadParams& p, cudaStream_t s) {
   const int Q = plan->Bp / 4;
   const size_t state = (size_t)plan->Bp * plan->geom.n * plan->geom.nsite * sizeof(float);
+  const Geometry& g = plan->geom;
+  const bool cube = g.L1 == 64 && g.L2 == 64 && g.L3 == 64 &&
+                    (plan->spec == Lat_bcc_1_2::id || plan->spec == Lat_fcc_1::id);
+  const unsigned ahead = cube ? kPrefetchBlocksCube : kPrefetchBlocks;
   for (int q0 = 0; q0 < Q; q0 += 65535) {
     p.q0 = q0;
     const int nq = Q - q0 < 65535 ? Q - q0 : 65535;
     const long long blocks = (long long)quad_blocks_x(plan) * nq;
-    p.ahead = state > kPrefetchState && blocks > 2 * kPrefetchBlocks ? kPrefetchBlocks : 0;
+    p.ahead = state > (cube ? kPrefetchStateCube : kPrefetchState) && blocks > 2 * ahead ? ahead : 0;
     launch_quad_grid(plan, p, dim3((unsigned)quad_blocks_x(plan), (unsigned)nq), s);
     const int rc = cuda_status(cudaGetLastError(), "interleaved class launch");
     if (rc != SCK_OK) return rc;

@@ -238,3 +238,20 @@ def test_topological_charge_of_any_block_size(Rd, layers, B):
         q = R.topological_charge(x[r:r + 1].contiguous(), 1)
         assert abs(float(Q[r]) - float(q[0])) < 3000 * 4 * np.pi * 2.0 ** -52
     assert float(Q.abs().max()) > 0
+
+
+@pytest.mark.parametrize("B", [21, 47])
+def test_interleaved_cube_of_four_classes_with_and_without_prefetch(B):
+    """The 64^3 cube of the J1-J2 lattice prefetches from 272 MB of state on: 151 MB and 302 MB, the last quad short."""
+    from spin_colour_kernel_b200 import workloads as wl
+    s = wl.heisenberg_bcc(64)
+    Q, R = (Sampler(s, B, device="cuda", seed=4, layout=layout) for layout in ("quad", "reference"))
+    R.tune(True, 0, 0)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn((B, 3) + s.shape, generator=g, device="cuda")
+    x /= x.norm(dim=1, keepdim=True)
+    X = Q.pack(x)
+    for A, Y in ((Q, X), (R, x)):
+        A.set_temperature(torch.linspace(0.5, 2.5, B))
+        A.sweep(Y, 1)
+    assert torch.equal(Q.unpack(X), x)
