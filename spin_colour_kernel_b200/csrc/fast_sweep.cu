@@ -185,13 +185,26 @@ __global__ void __launch_bounds__(256, 4) ising_march_kernel(const __grid_consta
   int ph = CUBIC ? first_class_x(c, p.colour, 0, y, z0) : first_class_x(c, p.colour, 0, z0, 0);
   uint32_t below = spin_codes(word((z0 > 0 ? z0 - 1 : len - 1) * step + row)), here = spin_codes(word(z0 * step + row));
   const uint32_t ctr0 = counter_of(rep, g.nsite, row);
+  // the next step's words are loaded ahead of this step's stores, past which the compiler may not move them
+  uint32_t w_above, w_ym = 0u, w_yp = 0u;
+  int8_t w_edge;
+  auto load = [&](int z, int p1) {
+    w_above = word((z + 1 < len ? z + 1 : 0) * step + row);
+    if constexpr (CUBIC) {
+      w_ym = word(z * step + ym);
+      w_yp = word(z * step + yp);
+    }
+    w_edge = src[z * step + (p1 ? right : left)];
+  };
+  load(z0, ph);
 #pragma unroll 2
   for (int z = z0; z < z1; ++z) {
     const int at = z * step;
-    const uint32_t above = spin_codes(word((z + 1 < len ? z + 1 : 0) * step + row));
+    const uint32_t above = spin_codes(w_above);
     uint32_t sum = below + above;
-    if constexpr (CUBIC) sum += spin_codes(word(at + ym)) + spin_codes(word(at + yp));
-    const uint32_t edge = (uint32_t)(1 + sgn(src[at + (ph ? right : left)]));
+    if constexpr (CUBIC) sum += spin_codes(w_ym) + spin_codes(w_yp);
+    const uint32_t edge = (uint32_t)(1 + sgn(w_edge));
+    if (z + 1 < z1) load(z + 1, ph ^ 1);
     const uint32_t even = here & 0x00FF00FFu, odd = (here >> 8) & 0x00FF00FFu;
     const uint32_t own = ph ? odd : even, other = ph ? even : odd;
     // neighbours along the row: the other residue's two, and one of them or the edge on the far side
