@@ -464,8 +464,9 @@ static int launch_tasks(const sck_plan* plan, SpecParams& p, cudaStream_t s) {
   }
   const uint32_t per = (uint32_t)p.c.rows * (uint32_t)p.c.bx;
   p.pairs = 1;
-  // up to four pairs a thread while eight blocks per SM are left: attempts/ns at one / two / four pairs, Heisenberg bcc
-  // J1-J2 64^3 x 2 x 64: 54 / 60 / 62; XY square 512^2 x 33: 108 / 127 / 144; Heisenberg sc 40^3 x 100: 75 / 79 / 84
+  // up to four pairs a thread while eight blocks per SM are left: attempts/ns at one / two / four pairs, XY square 512^2
+  // x 33: 116 / 142 / 166; Heisenberg sc 40^3 x 100: 82 / 89 / 92; bcc 32^3 x 64: 86 / 96 / 96; bcc J1-J2 64^3 x 2 x 64,
+  // whose 42 neighbour loads outweigh what pairs share: 64 / 63 / 62
   if (per_unit == 2)
     while (p.pairs < 4 && (long long)((per + 255) / 256) * p.n_tasks * ((most + 4 * p.pairs - 1) / (4 * p.pairs)) >= 148 * 8)
       p.pairs *= 2;

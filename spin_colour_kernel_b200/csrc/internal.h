@@ -30,7 +30,8 @@ struct Common {
   const float* beta;
   const void* table;
   const int64_t* state;
-  int sweep_offset;  // the launch's sweep is state[1] + sweep_offset (state advances once per call)
+  int sweep_offset;  // the launch's sweep is state[1] + sweep_offset: the lattice, word and interleaved kernels' state
+                     // advances once per call, the tile and generic kernels' every sweep (offset 0)
   int* giveup;       // the plan's host-mapped flag, raised (system scope) when a bounded wait gives up; may be null
   unsigned wait_limit;  // polls of a bounded wait before it gives up
   FastDiv fd_bx, fd_L1, fd_L2, fd_m[SCK_MAX_FACTORS];

@@ -249,11 +249,12 @@ __global__ void __launch_bounds__(128) weight_gradients_kernel(const __grid_cons
 }
 
 // ================================================================================ tcgen05 forward GEMM
-// C[M x N] = epilogue(A[M x K] B[N x K]^T) for the forward layers (both operands K-major), on the fifth-generation
-// tensor cores: a block of 128 threads owns 128 rows and all N columns; per 32-wide K chunk the threads stage
+// C[M x g.N] = epilogue(A[M x K] B[g.N x K]^T) for the forward layers (both operands K-major), on the fifth-generation
+// tensor cores: a block of 128 threads owns 128 rows and N columns (64, or a hidden layer's 256 for large batches); per
+// K chunk (half of the layer's inputs, 80 or 128 wide; 32 for large batches) the threads stage
 // A and B in shared memory in the canonical no-swizzle K-major layout (8-row x 16-byte core matrices: 128 bytes
-// apart along M or N, 16 x 128 bytes apart along K), one thread issues two tcgen05.mma (M 128, N, K 16, bf16
-// in, FP32 accumulating in tensor memory) and commits them to an mbarrier that all threads wait on (bounded)
+// apart along M or N, 16 x 128 bytes apart along K), one thread issues a tcgen05.mma per 16 of them (M 128, N, K 16,
+// bf16 in, FP32 accumulating in tensor memory) and commits them to an mbarrier that all threads wait on (bounded)
 // before the next chunk overwrites the stage. The epilogue reads the accumulator with tcgen05.ld (warp w reads
 // rows 32 w .. 32 w + 31) and applies bias, ReLU and the bfloat16 conversion.
 constexpr int UM = 128;     // rows per block (MMA M)
@@ -286,8 +287,9 @@ __device__ __forceinline__ bool umma_try_wait(uint32_t mbar, uint32_t parity) {
 
 // Grid (M / 128, g.N / N): a block multiplies one 128-row tile by N output columns. Its time is the latency of its
 // loads, so the 256-column layers run as four blocks of 64 columns per row tile: 256 blocks at M = 8192, all resident
-// at once, where 64 blocks of 256 columns left half of the SMs idle behind four times the copies each. K comes in two
-// chunks of KC, one per stage (eight of 32 put a copy's latency between every two products).
+// at once, where 64 blocks of 256 columns left half of the SMs idle behind four times the copies each. K then comes in two
+// chunks of KC, one per stage (eight of 32 put a copy's latency between every two products); umma_gemm gives the line
+// from which whole layers per block are the better ones.
 template <int N, int EPI, int KC>
 __global__ void __launch_bounds__(128) umma_gemm_kernel(GemmArgs g) {
   // two stages: the copies of chunk ch + 1 run while the tensor cores multiply chunk ch

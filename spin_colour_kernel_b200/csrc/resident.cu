@@ -423,6 +423,12 @@ int find_resident_spec(const sck_plan* plan) {
 }
 
 // Sweeps of a call from which the lists pay for their set-up (about a sweep's time), and their size in shared memory.
+// us constant offsets / lists: int8 square 64^2 x 148, 1 sweep 10.5 / 14.1, 2: 17.0 / 17.6, 3: 23.5 / 21.1, 4: 30.0 / 24.6,
+// 8: 55.8 / 38.7; Heisenberg bcc 8^3 x 148, 3: 12.3 / 13.2, 4: 15.1 / 15.6, 5: 17.7 / 17.8, 8: 25.9 / 24.8; nanodisk
+// 39 x 39 x 5 x 148, 1: 40.4 / 38.5, 4: 125 / 76. Lists take 16 or 32 bytes a site, which leaves fewer blocks to an
+// SM; in large batches they pay all the same from three or four sweeps on: int8 square 110^2 x 1,024 (one block
+// to an SM with lists), 3 sweeps 373 / 346, 4: 491 / 412; 64^2 x 1,024, 3: 135 / 119; Heisenberg fcc 8^3 x 1,024, 3: 126 / 131,
+// 4: 164 / 160.
 constexpr int kListSweeps = 4;
 constexpr size_t kResidentSmem = 222 << 10;
 
@@ -495,7 +501,9 @@ static int launch_lattice_resident_t(const sck_plan* plan, LatticeResidentParams
     LatticeResidentParams q = p;
     q.spin_bytes = (int)list_spin_bytes(plan);
     const size_t smem = list_bytes(plan);
-    // two blocks a replica when that still leaves a block to an SM and a class gives each block a round of threads
+    // two blocks a replica when that still leaves a block to an SM and a class gives each block a round of threads. Ten
+    // sweeps in us, one block / two: nanodisk 39 x 39 x 5 (3,808 sites a class) x 74 151 / 123, x 75 151 / 239; XY square 90^2
+    // x 74 97 / 73, 64^2 (2,048) 54 / 46, 56^2 (1,568) 46 / 42, 40^2 (800) 29 / 35
     if (N > 1 && 2 * B <= 148 && per >= 2048)
       return launch_resident_kernel(list_resident_kernel<Lat, N, ST, PER, (N > 1 ? 2 : 1)>, q, 2,
                                     block_threads((per + 1) / 2), smem, s);

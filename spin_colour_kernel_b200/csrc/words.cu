@@ -308,7 +308,7 @@ int find_word_spec(const sck_plan* plan) {
 // about two operations per pair. Only at the end of a column does the warp transpose the planes into one integer
 // per replica (warp_lane_counts), where the kernel for other systems (observables.cu) transposes every word of
 // every bond. Grid (blocks per word, words); a block takes the word's (column block, chunk) items in turn.
-// Bound by the logic pipe: 1083 -> 101 us for 128^3 x 512 replicas (1.3 TB/s of words), 40 -> 12 us for 64^3 x 128.
+// Bound by the logic pipe: 1083 -> 90 us for 128^3 x 512 replicas (1.5 TB/s of words), 40 -> 11 us for 64^3 x 128.
 constexpr int kPairPlanes = 11, kUpPlanes = 8;     // per-thread counters: chunks of at most 128 sites, 12 pairs each
 
 template <int N, int M>

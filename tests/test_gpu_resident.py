@@ -147,3 +147,16 @@ def test_marching_kernel_equals_the_generic_one(name, values):
         X.set_temperature(torch.linspace(1.5, 6.0, B))
         X.sweep(Y, 3)
     assert torch.equal(S, S2)
+
+
+def test_the_cases_above_run_on_the_kernels_they_are_for():
+    """Kind 7: lattice tables with neighbour lists; kind 1: the class kernel of boxes the marching kernel leaves."""
+    for name, build in RESIDENT.items():
+        s = build()
+        kw = dict(packed=False) if s.n == 1 else {}
+        A = Sampler(s, 5, device="cuda", **kw)
+        assert A.path()["specialised"] // 100 == 7, name
+        assert A.tune(False)["specialised"] == 0
+    for name in ["ising-square", "ising-sc-open", "ising-fcc", "ising-bcc-j1j2"]:
+        A = Sampler(RESIDENT[name](), 300, device="cuda", packed=False)
+        assert A.tune(True, 0, 0)["specialised"] // 100 == 1, name

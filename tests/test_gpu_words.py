@@ -87,3 +87,11 @@ def test_autotuning_words_times_the_word_kernels(tmp_path, monkeypatch):
     A.sweep(S, 3)
     R.sweep(S2, 3)
     assert torch.equal(S, S2)
+
+
+def test_the_systems_above_run_on_the_word_kernels():
+    for name in SYSTEMS:
+        for kw in (dict(packed=True), dict(bitwise=True), dict(bitwise=True, independent=True)):
+            A = Sampler(_system(name, 0.0, "metropolis"), 64, device="cuda", **kw)
+            assert A.path()["specialised"] // 100 == 5, name
+            assert A.tune(False)["specialised"] == 0
