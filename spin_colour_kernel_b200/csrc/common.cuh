@@ -76,7 +76,7 @@ __host__ __device__ __forceinline__ uint32_t fdiv(uint32_t n, FastDiv f) {
 // ---------------------------------------------------------------------------------------- dependent launches
 // Class launches of a sweep follow one another on a stream, each reading what the one before wrote. Launched with
 // launch_dependent (internal.h), a kernel's blocks may take their places while the last blocks of the one before
-// still run (launch_dependent asks for it where the grid's size makes it pay): every thread of such a kernel calls follow_previous before its first access to memory, which waits for
+// still run (launch_dependent with `overlap`): every thread of such a kernel calls follow_previous before its first access to memory, which waits for
 // the previous grid to finish with its writes visible, and lets the next one take its place. Loads after it are plain
 // (the compiler may move read-only loads across the wait).
 __device__ __forceinline__ void follow_previous() {

@@ -371,10 +371,23 @@ int find_spec(const sck_plan* p) {
 }
 
 // ------------------------------------------------------------------------------------------- host: launches
+// Grids of the vector class kernel that overlap the class before them: those of at most half a block per SM, of two to
+// two and a half blocks per SM, and of four fifths of the GPU's 740 places and more. Between these, the blocks that come early
+// share the SMs that the previous launch leaves room on, several to one while others stay empty, and the launch takes longer
+// than one that spreads over all SMs. Time of plain over overlapping launches, mean and range of 262 sweeps:
+//   blocks   up to 74    75-148     149-222    223-296    297-370    371-444    445-591    592-1,183  more
+//   mean     1.06        0.85       0.77       0.78       1.01       0.80       0.95       1.08       1.01-1.05
+//   range    0.96-1.18   0.68-1.02  0.65-0.92  0.67-1.04  0.94-1.10  0.76-0.88  0.90-1.03  1.04-1.12
+static bool overlap_pays(dim3 grid) {
+  constexpr long long kSms = 148, kPlaces = 5 * kSms;
+  const long long blocks = (long long)grid.x * grid.y;
+  return 2 * blocks <= kSms || (blocks > 2 * kSms && 2 * blocks <= 5 * kSms) || 5 * blocks >= 4 * kPlaces;
+}
+
 template <class Lat, int N, typename ST, bool PER, int NSL, class P>
 static void launch_one(const P& p, dim3 grid, cudaStream_t s) {
   if constexpr (std::is_same_v<P, SpecParams>)
-    launch_dependent(spec_task_kernel<Lat, N, PER, NSL>, grid, 256, 5, s, p);
+    launch_dependent(spec_task_kernel<Lat, N, PER, NSL>, grid, 256, s, p, overlap_pays(grid));
   else
     stream_kernel<Lat, N, ST, PER, NSL><<<grid, 256, 0, s>>>(p);
 }

@@ -155,21 +155,11 @@ int cuda_status(cudaError_t e, const char* where);
 
 // launchers (return SCK_OK or an error code)
 
-// A launch that may overlap the end of the stream's previous kernel; `kernel` calls follow_previous (common.cuh) and
-// runs `per_sm` blocks per SM. The overlap is asked for by grids of at most half a block per SM or of four fifths of the
-// places on the GPU and more. Between these, the blocks that come early share the SMs that the previous kernel leaves
-// room on, several to one while others stay empty, and a launch that would have spread over all SMs takes longer. Time of
-// plain over overlapping launches, means over 262 vector cases (five blocks per SM) and 276 of words (four and five):
-//   blocks        up to 37   to 74   to 148   to 296   to 444   to 592   to 888   to 1,184   more
-//   vector          1.03      1.07    0.85     0.78     0.86     0.95     1.08      1.07     1.01-1.05
-//   packed          1.17      1.05    0.76     0.93     0.92     1.10     1.08      1.05     1.01
-//   bitwise         1.19      1.13    0.91     0.87      -       0.99      -        1.06     1.06
-//   independent     1.15      1.04    0.80     0.90      -       1.09      -        1.05     1.03
+// A launch that may overlap the end of the stream's previous kernel; `kernel` calls follow_previous (common.cuh). Without
+// `overlap` it is a plain launch.
 template <class P>
-inline cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, unsigned threads, int per_sm, cudaStream_t s,
-                                    const P& p) {
-  constexpr long long kSms = 148;
-  const long long blocks = (long long)grid.x * grid.y * grid.z;
+inline cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, unsigned threads, cudaStream_t s, const P& p,
+                                    bool overlap = true) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -178,7 +168,7 @@ inline cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, unsigned threa
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 2 * blocks <= kSms || 5 * blocks >= 4 * kSms * per_sm ? 1 : 0;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 

@@ -350,7 +350,7 @@ int launch_unpack(const sck_plan* plan, const int32_t* words, const int8_t* mask
 }
 
 int launch_advance(int64_t* state, int n, cudaStream_t s) {
-  return cuda_status(launch_dependent(advance_kernel, dim3(1), 1, 1, s, AdvanceParams{state, n}), "advance");
+  return cuda_status(launch_dependent(advance_kernel, dim3(1), 1, s, AdvanceParams{state, n}), "advance");
 }
 
 }  // namespace sck

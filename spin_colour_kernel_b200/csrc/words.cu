@@ -502,11 +502,15 @@ int launch_word_columns(const sck_plan* plan, const ObsParams& p, cudaStream_t s
 }
 
 // --------------------------------------------------------------------------------------------- host side
+// Word launches overlap the class before them at every size. What they save, about a microsecond, is a fifth of a short
+// launch (packed fcc 18^3 x 37, 184 blocks: 4.9 us a class, 6.2 plain); where a grid crowds the SMs left over (one block
+// per SM in one launch of 75 to 148 blocks, two in the next) they lose more than that (packed fcc 10^3 x 256, 128
+// blocks: 6.0 us, 4.0 plain).
 template <class Lat, bool BARKER>
 static void launch_packed(const WordParams& p, int parts, dim3 grid, cudaStream_t s) {
-  if (parts == 1) launch_dependent(packed_lattice_kernel<Lat, 32, BARKER>, grid, 256, 4, s, p);
-  else if (parts == 2) launch_dependent(packed_lattice_kernel<Lat, 16, BARKER>, grid, 256, 4, s, p);
-  else launch_dependent(packed_lattice_kernel<Lat, 8, BARKER>, grid, 256, 4, s, p);
+  if (parts == 1) launch_dependent(packed_lattice_kernel<Lat, 32, BARKER>, grid, 256, s, p);
+  else if (parts == 2) launch_dependent(packed_lattice_kernel<Lat, 16, BARKER>, grid, 256, s, p);
+  else launch_dependent(packed_lattice_kernel<Lat, 8, BARKER>, grid, 256, s, p);
 }
 
 template <class Lat>
@@ -515,11 +519,11 @@ static void launch_word_t(const sck_plan* plan, const WordParams& p, int parts, 
     if (plan->geom.acceptance == SCK_BARKER) launch_packed<Lat, true>(p, parts, grid, s);
     else launch_packed<Lat, false>(p, parts, grid, s);
   } else if (plan->mode == SCK_MODE_BITWISE) {
-    if (p.c.field) launch_dependent(bitwise_shared_lattice_kernel<Lat, true>, grid, 256, 5, s, p);
-    else launch_dependent(bitwise_shared_lattice_kernel<Lat, false>, grid, 256, 5, s, p);
+    if (p.c.field) launch_dependent(bitwise_shared_lattice_kernel<Lat, true>, grid, 256, s, p);
+    else launch_dependent(bitwise_shared_lattice_kernel<Lat, false>, grid, 256, s, p);
   } else {
-    if (p.c.field) launch_dependent(bitwise_independent_lattice_kernel<Lat, true>, grid, 256, 4, s, p);
-    else launch_dependent(bitwise_independent_lattice_kernel<Lat, false>, grid, 256, 4, s, p);
+    if (p.c.field) launch_dependent(bitwise_independent_lattice_kernel<Lat, true>, grid, 256, s, p);
+    else launch_dependent(bitwise_independent_lattice_kernel<Lat, false>, grid, 256, s, p);
   }
 }
 
