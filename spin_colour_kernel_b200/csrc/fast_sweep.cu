@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256, 4) ising_march_kernel(const __grid_consta
     uint32_t sum = below + above;
     if constexpr (CUBIC) sum += spin_codes(w_ym) + spin_codes(w_yp);
     const uint32_t edge = (uint32_t)(1 + sgn(w_edge));
-    if (z + 1 < z1) load(z + 1, ph ^ 1);
+    load(min(z + 1, z1 - 1), ph ^ 1);
     const uint32_t even = here & 0x00FF00FFu, odd = (here >> 8) & 0x00FF00FFu;
     const uint32_t own = ph ? odd : even, other = ph ? even : odd;
     // neighbours along the row: the other residue's two, and one of them or the edge on the far side
@@ -519,8 +519,8 @@ static void launch_ising_t(const sck_plan* plan, const IsingClassParams& p, dim3
 //   filled:  square 4 x 60,000 x 100 (1 word of 256) 129 / 4,425; 256 x 1,024 x 33 (64) 50.2 / 57.8;
 //            500^2 x 33 (125) 48.6 / 45.4; 1,024 x 256 x 33 (256) 50.2 / 44.6
 //   walks:   sc 64^3 x 1 (8,192) 7.6 / 14.0, x 3 (24,576) 14.7 / 15.1, x 4 (32,768) 18.1 / 15.2; sc 96^3 x 1 (27,648)
-//            15.8 / 14.4; square 512^2 x 3 (24,576) 13.4 / 13.6, x 4 (32,768) 16.4 / 13.9
-constexpr long long kMarchWalks = 26000;
+//            15.8 / 14.4; square 512^2 x 2 (16,384) 10.6 / 10.9, x 3 (24,576) 13.4 / 11.7
+constexpr long long kMarchWalks = 26000, kMarchWalks2 = 20000;   // three dimensions, two
 
 bool ising_march_plan(const sck_plan* plan) {
   const Geometry& g = plan->geom;
@@ -532,7 +532,7 @@ bool ising_march_plan(const sck_plan* plan) {
     if (col.K[0][k] != 1) return false;
   const int cols = g.L1 / 4 * (g.dim == 3 ? g.L2 : 1), len = g.dim == 3 ? g.L3 : g.L2;
   if (16 * (long long)cols < 7 * 256 * (long long)((cols + 255) / 256)) return false;
-  return (long long)cols * ((len + 7) / 8) * plan->Bp >= kMarchWalks;
+  return (long long)cols * ((len + 7) / 8) * plan->Bp >= (g.dim == 3 ? kMarchWalks : kMarchWalks2);
 }
 
 // Its 4-byte loads need spins that start on 4 bytes.

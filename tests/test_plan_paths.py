@@ -113,6 +113,7 @@ def test_marching_kernel_takes_full_blocks_and_enough_walks():
     for crystal, box, B, kind in (("square", (4, 60000), 100, 1), ("square", (256, 1024), 100, 1),
                                   ("square", (500, 500), 33, 8), ("square", (1024, 256), 8, 8), ("sc", (16, 4, 4000), 33, 1),
                                   ("sc", (64, 64, 64), 1, 1), ("sc", (64, 64, 64), 3, 1), ("sc", (64, 64, 64), 4, 8),
-                                  ("sc", (96, 96, 96), 1, 8), ("sc", (32, 32, 256), 100, 8)):
+                                  ("sc", (96, 96, 96), 1, 8), ("sc", (32, 32, 256), 100, 8),
+                                  ("square", (512, 512), 2, 1), ("square", (512, 512), 3, 8)):
         A = plan_of(_box(crystal, box), B, L.MODE_INT8)
         assert A.path()["specialised"] // 100 == kind, (box, B, A.path())
